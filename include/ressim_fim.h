@@ -244,8 +244,10 @@ int32_t rf_set_cluster_size(RfCtx* ctx, int32_t ctas);
  * vectors in level order and the sweeps' dependencies in shared memory (`threads` threads,
  * 32..512 in steps of 32, 0 automatic); RF_PRESSURE_SOLVER_AUTO (default) takes the level-order
  * kernels, where their level window fits shared memory, for decks of up to 32,768 cells and for
- * every variant of an ensemble stepped in RF_BATCH_GROUPS mode, and the cluster kernels otherwise.  Both compute the same preconditioner;
- * the solves differ only in the summation order of their dot products.  Takes effect at the next
+ * every variant of an ensemble stepped in RF_BATCH_GROUPS mode, and the cluster kernels otherwise;
+ * its pressure BiCGStab runs along grid lines where the deck allows, with the results of the kernel
+ * it stands in for bit for bit.  All compute the same preconditioner; the cluster's and the level
+ * order's solves differ only in the summation order of their dot products.  Takes effect at the next
  * linear solve; RF_ERR_UNSUPPORTED when the level-order kernels cannot run this deck.  No
  * counterpart in the reference. */
 #define RF_PRESSURE_SOLVER_AUTO 0

@@ -1185,6 +1185,7 @@ static void free_ctx(Ctx& c) {
   c.d_dir_perm.free();
   c.dir_rows = 0;
   free_level_plan(c);
+  free_pencil_plan(c);
   for (auto* b : {&c.d_tri_ptr, &c.d_tri_up, &c.d_tri_ip, &c.d_pt_ptr, &c.d_pt_lp, &c.d_pt_ue}) b->free();
   c.d_ref_b.free();
   c.d_fac_simple.free();
@@ -1677,11 +1678,18 @@ int32_t regroup(RfBatch* b, int mode) {
       c.stream_owned = 1;
     }
     c.batched = 0;
+    c.ensemble = int(b->ctx.size());
   }
   for (auto& g : b->groups)
     if (g->stream) cudaStreamDestroy(g->stream);
   b->groups.clear();
   b->mode = mode;
+  struct Replan {  // on every way out
+    RfBatch* b;
+    ~Replan() {
+      for (RfCtx* x : b->ctx) rf::pencil_replan(x->c);
+    }
+  } replan{b};
   if (mode != RF_BATCH_GROUPS) return RF_OK;
   const int n = int(b->ctx.size());
   const int G = std::max(1, std::min(b->threads, n));

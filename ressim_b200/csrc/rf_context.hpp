@@ -4,8 +4,10 @@
 
 #include <cuda_runtime.h>
 
+#include <set>
 #include <string>
 #include <cstring>
+#include <utility>
 #include <vector>
 
 #include "../../include/ressim_fim.h"
@@ -98,6 +100,29 @@ struct LevelPlan {
   size_t blk_smem[2] = {0, 0};
 };
 
+// Plan of the pressure BiCGStab whose sweeps run along grid lines on a cluster (rf_pencil.cu):
+// the rows outside the 7-point shape, and the step-order layout for `cs` CTAs.
+struct PencilPlan {
+  int built = 0;
+  int fits[2][5] = {};   // per value type (0 double, 1 float): runs on 1, 2, 4, 8, 16 CTAs (-1: not asked yet)
+  int chunk[2][5] = {};  // and the steps whose rows it copies at a time
+  int cs = 0;           // CTAs the layout is for (0: none)
+  int slots = 0, n_spec_entries = 0, n_well_entries = 0;
+  int packed = -1;      // value type of the last packing (-1: none since the last factorisation)
+  struct Listed {
+    int j, entries;
+  };
+  std::vector<Listed> listed;               // rows taken from lists: column, entries off the diagonal
+  std::set<std::pair<int, int>> fill_cols;  // columns (j, j') joined by a well's fill
+  std::vector<int> h_spec_row, h_spec_col_row, h_nat, dots_key;  // dots_key: the order d_list holds
+  DBuf<int> d_cta, d_nat, d_rec_at, d_rec_half, d_list_ptr, d_list[3], d_spec_slot, d_spec_ptr, d_spec_col, d_spec_map;
+  DBuf<int> d_well_cta, d_well_at, d_well_slot, d_well_ptr, d_well_row, d_well_map;
+  DBuf<unsigned short> d_well_code;
+  // values, sized for double and holding either type
+  DBuf<double> d_well_val, d_well_piv, d_spec_val, d_lrec, d_brec, d_arec, d_rd;
+  DBuf<unsigned char> d_special, d_work;
+};
+
 // Cooperative scheduling of an ensemble's variants on shared host threads (rf_fiber.cu).  Inside a
 // batch step each variant's controller runs as a fiber on its group's thread: a wait on the
 // stream suspends the fiber instead of blocking the thread, and the level-scheduled kernels of the
@@ -110,6 +135,7 @@ struct Ctx {
   cudaStream_t stream = nullptr;
   int stream_owned = 1;  // 0: the stream belongs to an ensemble group (rf_batch_create)
   int batched = 0;       // the context's level-scheduled kernels join its group's batched launches
+  int ensemble = 0;      // variants of the ensemble the context belongs to (0: none)
   cudaEvent_t ev_wait = nullptr;  // stream waits of a fiber
   long long launches = 0;
   int device = 0, num_sms = 0;
@@ -232,6 +258,7 @@ struct Ctx {
   int pressure_solver = 0;
   int level_threads = 0;  // threads of the level-order kernels (0: automatic)
   LevelPlan lvl;
+  PencilPlan pen;
 
   // timing
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;

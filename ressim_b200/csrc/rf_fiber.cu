@@ -67,7 +67,7 @@ void suspend(int state) {
 void launch_pending(BatchGroup& g) {
   std::vector<BatchItem>& items = g.pending;
   for (int kind = 0; kind < kBatchKinds; ++kind)
-    for (int type = 0; type < 2; ++type) {
+    for (int type = 0; type < kBatchTypes; ++type) {
       std::vector<const BatchItem*> sel;
       for (const BatchItem& it : items)
         if (it.kind == kind && it.type == type) sel.push_back(&it);

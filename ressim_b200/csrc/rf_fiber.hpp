@@ -15,13 +15,15 @@ constexpr int kBatchPressure = 0;
 constexpr int kBatchBlockSweep = 1;
 constexpr int kBatchFactor = 2;
 constexpr int kBatchKinds = 3;
+constexpr int kBatchTypes = 12;  // values of BatchItem::type
 // Items per launch: the kernel parameter carries their arguments by value.
 constexpr int kBatchItems = 24;
 constexpr size_t kBatchArgBytes = 320;
 
 struct BatchItem {
   int kind = 0;
-  int type = 0;  // 0 double, 1 float
+  int type = 0;  // value type: 0 double, 1 float; the pressure solve along lines adds 2 (1 + log2 of
+                 // its cluster size), so a launch's items share one cluster size
   int threads = 0;
   size_t smem = 0;
   alignas(16) unsigned char args[kBatchArgBytes];
@@ -61,5 +63,7 @@ void run_fibers(BatchGroup& g, void (*fn)(void*), void* const* args, int count, 
 bool launch_batch_items(int kind, int type, const BatchItem* const* items, int count, cudaStream_t stream);
 // The factorisation's batched launch (rf_linear.cu).
 bool launch_factor_batch(const BatchItem* const* items, int count, cudaStream_t stream);
+// The batched launch of the pressure solve along lines (rf_pencil.cu).
+bool launch_pencil_batch(int type, const BatchItem* const* items, int count, cudaStream_t stream);
 
 }  // namespace rf

@@ -1079,6 +1079,7 @@ static bool launch_batch(const BatchItem* const* items, int count, cudaStream_t 
 bool launch_batch_items(int kind, int type, const BatchItem* const* items, int count, cudaStream_t stream) {
   if (count <= 0) return true;
   if (kind == kBatchFactor) return launch_factor_batch(items, count, stream);
+  if (kind == kBatchPressure && type >= 2) return launch_pencil_batch(type, items, count, stream);
   if (kind == kBatchPressure) {
     if (type == 1)
       return launch_batch<LvlArgs<float>, LvlBatch<float>>(items, count, stream,

@@ -2266,9 +2266,28 @@ static void cpr_build(Ctx& c) {
     cluster_launch(c, (const void*)k_factor_cluster, kFBlock, args);
   }
   c.lvl.packed = -1;
-  const bool level = level_solver_active(c);
+  c.pen.packed = -1;
+  if (c.precision == 1) {
+    k_factors_to_f32<<<4 * c.num_sms, kBlock, 0, c.stream>>>(
+        9ll * c.nnzb, c.d_lu.p, c.d_lu32.p, 9ll * n, c.d_dinv.p, c.d_dinv32.p, c.nnzb, c.d_plu.p, c.d_plu32.p,
+        c.d_pval.p, c.d_pval32.p, n, c.d_pdiag.p, c.d_pdiag32.p);
+    c.launches++;
+  }
+  c.dense_ok = 0;
+  if (n <= kDenseCoarseCells) {
+    k_dense_build<<<blocks_for(n), kBlock, 0, c.stream>>>(n, c.d_row_ptr.p, c.d_col.p, c.d_pval.p, c.d_tmp2.p);
+    dense_invert_launch(n, c.d_tmp2.p, c.d_dense.p, c.d_dense_perm.p, c.d_flag_dense.p, c.stream);
+    c.launches += 2;
+    int ok = 0;
+    d2h(c, &ok, c.d_flag_dense.p, sizeof(int));
+    d2h_wait(c);
+    c.dense_ok = ok;
+  }
+  if (c.dense_ok) return;
+  const bool lines = pencil_active(c), level = !lines && level_solver_active(c);
+  if (lines) pencil_pack(c);
   if (level) level_pack(c);
-  if (!level && c.dsm_bytes[c.precision == 1 ? 1 : 0] != 0) {
+  if (!lines && !level && c.dsm_bytes[c.precision == 1 ? 1 : 0] != 0) {
     if (c.precision == 1)
       k_pack_sweeps<float><<<blocks_for(n), kBlock, 0, c.stream>>>(n, c.d_own_rows.p, c.d_row_ptr.p, c.d_diag.p,
                                                                    c.d_fcnt.p, c.d_bcnt.p, c.d_plu.p, c.d_pdiag.p,
@@ -2278,22 +2297,6 @@ static void cpr_build(Ctx& c) {
                                                                     c.d_fcnt.p, c.d_bcnt.p, c.d_plu.p, c.d_pdiag.p,
                                                                     c.d_fval.p, c.d_bval.p, c.d_dval.p);
     c.launches++;
-  }
-  if (c.precision == 1) {
-    k_factors_to_f32<<<4 * c.num_sms, kBlock, 0, c.stream>>>(
-        9ll * c.nnzb, c.d_lu.p, c.d_lu32.p, 9ll * n, c.d_dinv.p, c.d_dinv32.p, c.nnzb, c.d_plu.p, c.d_plu32.p,
-        c.d_pval.p, c.d_pval32.p, n, c.d_pdiag.p, c.d_pdiag32.p);
-    c.launches++;
-  }
-  c.dense_ok = 0;
-  if (n <= 299) {
-    k_dense_build<<<blocks_for(n), kBlock, 0, c.stream>>>(n, c.d_row_ptr.p, c.d_col.p, c.d_pval.p, c.d_tmp2.p);
-    dense_invert_launch(n, c.d_tmp2.p, c.d_dense.p, c.d_dense_perm.p, c.d_flag_dense.p, c.stream);
-    c.launches += 2;
-    int ok = 0;
-    d2h(c, &ok, c.d_flag_dense.p, sizeof(int));
-    d2h_wait(c);
-    c.dense_ok = ok;
   }
 }
 
@@ -2361,9 +2364,21 @@ static bool launch_bicgstab_dsmem(Ctx& c, const T* pval, const T* plu, const T* 
   return true;
 }
 
+// Summation order of the dot products of the level-list kernel the pressure solve would take.
+PencilDots pressure_dots(const Ctx& c) {
+  const int f = c.precision == 1 ? 1 : 0;
+  if (level_solver_active(c)) return {0, c.lvl.threads[f], 1, 0};
+  if (c.dsm_bytes[f] != 0) return {1, kDBlock, c.cluster_size, c.own_slice};
+  return {2, kCBlock, c.cluster_size, 0};
+}
+
 template <class T>
 static void launch_bicgstab(Ctx& c, const T* pval, const T* plu, const T* pdiag, const double* rhs, double* x,
                             T* base) {
+  if (pencil_active(c)) {
+    launch_bicgstab_pencil(c, rhs, x);
+    return;
+  }
   if (level_solver_active(c)) {
     launch_bicgstab_level(c, rhs, x);
     return;
@@ -3074,6 +3089,7 @@ void set_linear_precision(Ctx& c, int mode) {
     c.d_sweep32.alloc(6 * n);
   }
   c.precision = mode;
+  pencil_replan(c);
 }
 
 void setup_linear_workspace(Ctx& c) {
@@ -3108,6 +3124,7 @@ void setup_linear_workspace(Ctx& c) {
   // the largest cluster (16 CTAs, non-portable; else 8) that every level-scheduled kernel can run
   set_cluster_size(c, auto_cluster_size(c));
   build_level_plan(c);
+  build_pencil_plan(c);
   build_factor_recipes(c);
   const int nt = 1 + c.topo.max_perfs_per_well;
   const size_t smem = sizeof(double) * (2 * size_t(nt) * nt + 2 * nt);

@@ -95,4 +95,22 @@ void level_pack(Ctx& c);
 void launch_bicgstab_level(Ctx& c, const double* rhs, double* x);
 void launch_block_sweep_level(Ctx& c, const double* cr, double* x, const void* lu, const void* dinv);
 
+// Largest deck whose pressure stage is the dense inverse of its matrix.
+constexpr int kDenseCoarseCells = 299;
+
+// The pressure BiCGStab along grid lines (rf_pencil.cu): in automatic mode, wherever the deck
+// allows, it takes the place of the level-order or cluster kernel with that kernel's summation order.
+struct PencilDots {
+  int kind;     // 0 level order, 1 cluster in slices, 2 cluster grid-strided
+  int threads;  // per block
+  int blocks, slice;
+};
+void build_pencil_plan(Ctx& c);
+void pencil_replan(Ctx& c);
+void free_pencil_plan(Ctx& c);
+bool pencil_active(const Ctx& c);
+void pencil_pack(Ctx& c);
+void launch_bicgstab_pencil(Ctx& c, const double* rhs, double* x);
+PencilDots pressure_dots(const Ctx& c);
+
 }  // namespace rf

@@ -169,7 +169,7 @@ class ReservoirSimulator(Deck):
     def set_pressure_solver(self, kind: str = "auto", threads: int = 0) -> None:
         """Kernels of the CPR's level-scheduled solves: "cluster" (the thread-block cluster
         kernels), "level" (one thread block in level order, `threads` threads, 0 automatic) or
-        "auto"."""
+        "auto" (one of these by size, the pressure solve along grid lines where the deck allows)."""
         codes = {"auto": 0, "cluster": 1, "level": 2}
         if kind not in codes:
             raise ValueError(f"pressure solver must be one of {sorted(codes)}")
