@@ -13,7 +13,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "_build")
 OUT = os.path.join(HERE, "libressim_fim.so")
-SOURCES = ["rf_assembly.cu", "rf_linear.cu", "rf_direct.cu", "rf_state.cu", "rf_api.cu", "rf_noalloc.cu",
+SOURCES = ["rf_assembly.cu", "rf_linear.cu", "rf_factor.cu", "rf_direct.cu", "rf_state.cu", "rf_api.cu", "rf_noalloc.cu",
            "rf_blackoil.cu", "rf_adjoint.cu", "rf_level.cu",
            "rf_pencil.cu", "rf_fiber.cu"]
 COMPILE_FLAGS = [

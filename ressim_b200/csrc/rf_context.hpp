@@ -123,6 +123,15 @@ struct PencilPlan {
   DBuf<unsigned char> d_special, d_work;
 };
 
+// Plan of the ILU0 factorisations (rf_factor.cu): simple rows and listed rows' steps by level.
+struct FactorPlan {
+  int built = 0, cs = 1;  // cs: CTAs of a single deck's factorisation
+  DBuf<int> d_row_ptr, d_step_ptr;
+  DBuf<int4> d_rec, d_step, d_entry;
+  DBuf<int2> d_pair;
+  DBuf<unsigned char> d_simple;  // [n]
+};
+
 // Cooperative scheduling of an ensemble's variants on shared host threads (rf_fiber.cu).  Inside a
 // batch step each variant's controller runs as a fiber on its group's thread: a wait on the
 // stream suspends the fiber instead of blocking the thread, and the level-scheduled kernels of the
@@ -251,9 +260,7 @@ struct Ctx {
   int precision = 0;
   DBuf<float> d_lu32, d_dinv32, d_plu32, d_pval32, d_pdiag32, d_pvec32, d_sweep32;
   DBuf<int> d_flag_dense;
-  // update lists of the factorisation (rf_linear.cu, FacRecipes)
-  DBuf<int> d_tri_ptr, d_tri_up, d_tri_ip, d_pt_ptr, d_pt_lp, d_pt_ue;
-  DBuf<unsigned char> d_fac_simple;  // [n] rows of the simple shape (rf_linear.cu, ilu_row_simple)
+  FactorPlan fac;
   // pressure-stage solver: 0 automatic, 1 the cluster kernels, 2 the single-CTA level-order kernels
   int pressure_solver = 0;
   int level_threads = 0;  // threads of the level-order kernels (0: automatic)

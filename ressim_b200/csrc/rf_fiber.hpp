@@ -10,7 +10,7 @@
 namespace rf {
 
 // Kinds of batched launches: the pressure BiCGStab and the block-ILU0 sweep (rf_level.cu), the
-// block-ILU0 and pressure-ILU0 factorisation (rf_linear.cu).
+// block-ILU0 and pressure-ILU0 factorisation (rf_factor.cu).
 constexpr int kBatchPressure = 0;
 constexpr int kBatchBlockSweep = 1;
 constexpr int kBatchFactor = 2;
@@ -61,7 +61,7 @@ void run_fibers(BatchGroup& g, void (*fn)(void*), void* const* args, int count, 
 // One launch of `count` items of one kind and value type on `stream` (rf_level.cu); false when
 // the launch failed.
 bool launch_batch_items(int kind, int type, const BatchItem* const* items, int count, cudaStream_t stream);
-// The factorisation's batched launch (rf_linear.cu).
+// The factorisation's batched launch (rf_factor.cu).
 bool launch_factor_batch(const BatchItem* const* items, int count, cudaStream_t stream);
 // The batched launch of the pressure solve along lines (rf_pencil.cu).
 bool launch_pencil_batch(int type, const BatchItem* const* items, int count, cudaStream_t stream);

@@ -26,48 +26,12 @@
 #include <cstdio>
 
 #include "rf_fiber.hpp"
+#include "rf_mat3.cuh"
 #include "rf_ops.hpp"
 
 namespace rf {
 
 constexpr double kEps = kF64Eps;
-
-// ============================================================================================
-// small dense helpers
-// ============================================================================================
-__device__ __forceinline__ void mat3_mul(const double* a, const double* b, double* c) {
-#pragma unroll
-  for (int r = 0; r < 3; ++r)
-#pragma unroll
-    for (int k = 0; k < 3; ++k) c[3 * r + k] = a[3 * r] * b[k] + a[3 * r + 1] * b[3 + k] + a[3 * r + 2] * b[6 + k];
-}
-// 3x3 inverse by cofactors; fails only on an exactly zero determinant, then the diagonal
-// reciprocal fallback (gmres_block_jacobi.rs:888-901) is used.
-__host__ __device__ __forceinline__ void mat3_inverse_or_diag(const double* m, double* o) {
-  const double m11 = m[0], m12 = m[1], m13 = m[2], m21 = m[3], m22 = m[4], m23 = m[5], m31 = m[6], m32 = m[7],
-               m33 = m[8];
-  const double c11 = m22 * m33 - m32 * m23;
-  const double c21 = m21 * m33 - m31 * m23;
-  const double c31 = m21 * m32 - m31 * m22;
-  const double det = m11 * c11 - m12 * c21 + m13 * c31;
-  if (det != 0.0) {
-    o[0] = c11 / det;
-    o[1] = (m13 * m32 - m33 * m12) / det;
-    o[2] = (m12 * m23 - m22 * m13) / det;
-    o[3] = -c21 / det;
-    o[4] = (m11 * m33 - m31 * m13) / det;
-    o[5] = (m13 * m21 - m23 * m11) / det;
-    o[6] = c31 / det;
-    o[7] = (m12 * m31 - m32 * m11) / det;
-    o[8] = (m11 * m22 - m21 * m12) / det;
-    return;
-  }
-  for (int k = 0; k < 9; ++k) o[k] = 0.0;
-  for (int d = 0; d < 3; ++d) {
-    const double v = m[4 * d];
-    o[4 * d] = fabs(v) > kEps ? 1.0 / v : 1.0;
-  }
-}
 
 // ============================================================================================
 // BSR SpMV and vector kernels
@@ -757,21 +721,6 @@ __device__ __forceinline__ const int* stage_levels(const LevelSched& L, int* s_p
   return L.lvl_ptr;
 }
 
-// Precomputed update lists of the factorisation (built once per pattern): for each lower entry kp
-// of a row, the pairs (up, ip) of the U-row of col[kp] whose column the row also holds (the
-// merge block_ilu_row performs); for each entry k of a row, the terms (lp, ue) of the pressure ILU
-// (pressure_ilu_row's lower entries lp before it whose row holds the column of k above its
-// diagonal, at entry ue).  Present-entry checks on the values stay at run time.
-struct FacRecipes {
-  const int* tri_ptr;  // [nnzb + 1]
-  const int* tri_up;
-  const int* tri_ip;
-  const int* pt_ptr;   // [nnzb + 1]
-  const int* pt_lp;
-  const int* pt_ue;
-  const unsigned char* simple;  // [n] 1: the row takes ilu_row_simple
-};
-
 struct FacArgs {
   LevelSched L;
   const double* val;
@@ -781,389 +730,30 @@ struct FacArgs {
   const double* pval;
   double* plu;
   double* pdiag;
-  FacRecipes R;  // tri_ptr == nullptr: search as block_ilu_row / pressure_ilu_row do
 };
 
-// Both ILU0 rows of row i from the update lists: the same operations in the same order as
-// block_ilu_row and pressure_ilu_row.
-__device__ void ilu_row_recipe(int i, const FacArgs& a) {
-  const int* rp = a.L.rp;
-  const int* col = a.L.col;
-  const int b0 = rp[i], dp = a.L.diag[i], b1 = rp[i + 1];
-  const FacRecipes& R = a.R;
-  for (int k = b0; k < b1; ++k) {
-    const bool m = a.mask[k];
-    for (int e = 0; e < 9; ++e) a.lu[size_t(k) * 9 + e] = m ? a.val[size_t(k) * 9 + e] : 0.0;
-  }
-  for (int kp = b0; kp < dp; ++kp) {
-    if (!a.mask[kp]) continue;
-    double lik[9];
-    mat3_mul(a.lu + size_t(kp) * 9, a.dinv + size_t(col[kp]) * 9, lik);
-    for (int e = R.tri_ptr[kp]; e < R.tri_ptr[kp + 1]; ++e) {
-      const int up = R.tri_up[e], ip = R.tri_ip[e];
-      if (!a.mask[up] || !a.mask[ip]) continue;
-      double prod[9];
-      mat3_mul(lik, a.lu + size_t(up) * 9, prod);
-      double* t = a.lu + size_t(ip) * 9;
-      for (int q = 0; q < 9; ++q) t[q] -= prod[q];
-    }
-    for (int q = 0; q < 9; ++q) a.lu[size_t(kp) * 9 + q] = lik[q];
-  }
-  mat3_inverse_or_diag(a.lu + size_t(dp) * 9, a.dinv + size_t(i) * 9);
-  // pressure ILU0
-  auto terms = [&](int k, double s) {
-    for (int e = R.pt_ptr[k]; e < R.pt_ptr[k + 1]; ++e) {
-      const int lp = R.pt_lp[e];
-      if (a.pval[lp] == 0.0) continue;
-      s -= a.plu[lp] * a.plu[R.pt_ue[e]];
-    }
-    return s;
-  };
-  for (int kp = b0; kp < dp; ++kp) {
-    if (a.pval[kp] == 0.0) {
-      a.plu[kp] = 0.0;
-      continue;
-    }
-    const double s = terms(kp, a.pval[kp]);
-    const double d = a.pdiag[col[kp]];
-    a.plu[kp] = fabs(d) > kEps ? s / d : 0.0;
-  }
-  const double de = a.pval[dp];
-  double ud = terms(dp, de);
-  if (fabs(ud) <= kEps) ud = fabs(de) > kEps ? de : 1.0;
-  a.pdiag[i] = ud;
-  a.plu[dp] = 0.0;
-  for (int up = dp + 1; up < b1; ++up) {
-    if (a.pval[up] == 0.0) {
-      a.plu[up] = 0.0;
-      continue;
-    }
-    a.plu[up] = terms(up, a.pval[up]);
-  }
-}
-// Both ILU0 rows of a "simple" row, the shape of every 7-point stencil row: at most kSimpleLower
-// lower entries, each updating only the diagonal block (at most one pair per lower entry, its
-// target the diagonal), and pressure terms only on the diagonal.  Then no lower entry changes
-// before it is used, so the row's inputs (its own values, the lower columns' inverse diagonal
-// blocks and pivots, the U blocks and pressure factors the updates read) are all loaded first, in
-// a few independent rounds, instead of the chain of dependent loads the general walk takes.  The
-// arithmetic is ilu_row_recipe's, in its order: L_ik = lu_kp Dinv_col[kp], the diagonal minus
-// L_ik U_up in kp order, the pressure lower entries s / d, the diagonal's terms in list order.
-constexpr int kSimpleLower = 4;
-__device__ void ilu_row_simple(int i, const FacArgs& a) {
-  const int* rp = a.L.rp;
-  const int* col = a.L.col;
-  const FacRecipes& R = a.R;
-  const int b0 = __ldg(rp + i), dp = __ldg(a.L.diag + i), b1 = __ldg(rp + i + 1);
-  const int nl = dp - b0;
-  // structure (read-only in this kernel)
-  int ck[kSimpleLower], up[kSimpleLower];
-  bool mk[kSimpleLower];
-  double pv[kSimpleLower];
-#pragma unroll
-  for (int j = 0; j < kSimpleLower; ++j) {
-    ck[j] = 0;
-    up[j] = -1;
-    mk[j] = false;
-    pv[j] = 0.0;
-    if (j < nl) {
-      const int k = b0 + j;
-      ck[j] = __ldg(col + k);
-      mk[j] = __ldg(a.mask + k) != 0;
-      pv[j] = __ldg(a.pval + k);
-      const int e0 = __ldg(R.tri_ptr + k), e1 = __ldg(R.tri_ptr + k + 1);
-      if (e1 > e0) up[j] = __ldg(R.tri_up + e0);
-    }
-  }
-  const bool md = __ldg(a.mask + dp) != 0;
-  double D[9];
-#pragma unroll
-  for (int e = 0; e < 9; ++e) D[e] = md ? __ldg(a.val + size_t(dp) * 9 + e) : 0.0;
-  // block ILU0: each present lower entry's L_ik, and its update of the diagonal in kp order; the
-  // row's stores wait until all its loads are issued
-  double lik[kSimpleLower][9];
-#pragma unroll
-  for (int j = 0; j < kSimpleLower; ++j) {
-#pragma unroll
-    for (int e = 0; e < 9; ++e) lik[j][e] = 0.0;
-    if (j >= nl || !mk[j]) continue;
-    const int k = b0 + j;
-    double lk[9], dk[9];
-#pragma unroll
-    for (int e = 0; e < 9; ++e) {
-      lk[e] = __ldg(a.val + size_t(k) * 9 + e);
-      dk[e] = a.dinv[size_t(ck[j]) * 9 + e];
-    }
-    mat3_mul(lk, dk, lik[j]);
-    if (up[j] >= 0 && md && __ldg(a.mask + up[j])) {
-      double u[9], prod[9];
-#pragma unroll
-      for (int e = 0; e < 9; ++e) u[e] = a.lu[size_t(up[j]) * 9 + e];
-      mat3_mul(lik[j], u, prod);
-#pragma unroll
-      for (int e = 0; e < 9; ++e) D[e] -= prod[e];
-    }
-  }
-#pragma unroll
-  for (int j = 0; j < kSimpleLower; ++j)
-    if (j < nl) {
-#pragma unroll
-      for (int e = 0; e < 9; ++e) a.lu[size_t(b0 + j) * 9 + e] = lik[j][e];
-    }
-  for (int k = dp + 1; k < b1; ++k) {
-    const bool m = __ldg(a.mask + k) != 0;
-#pragma unroll
-    for (int e = 0; e < 9; ++e) a.lu[size_t(k) * 9 + e] = m ? __ldg(a.val + size_t(k) * 9 + e) : 0.0;
-  }
-#pragma unroll
-  for (int e = 0; e < 9; ++e) a.lu[size_t(dp) * 9 + e] = D[e];
-  mat3_inverse_or_diag(D, a.dinv + size_t(i) * 9);
-  // pressure ILU0: lower entries (no terms), the diagonal's terms in list order, upper entries
-  double pl[kSimpleLower];
-#pragma unroll
-  for (int j = 0; j < kSimpleLower; ++j) {
-    pl[j] = 0.0;
-    if (j < nl && pv[j] != 0.0) {
-      const double d = a.pdiag[ck[j]];
-      pl[j] = fabs(d) > kEps ? pv[j] / d : 0.0;
-    }
-    if (j < nl) a.plu[b0 + j] = pl[j];
-  }
-  const double de = __ldg(a.pval + dp);
-  double ud = de;
-  for (int e = __ldg(R.pt_ptr + dp); e < __ldg(R.pt_ptr + dp + 1); ++e) {
-    const int jl = __ldg(R.pt_lp + e) - b0;
-    double plp = 0.0, pvl = 0.0;
-#pragma unroll
-    for (int j = 0; j < kSimpleLower; ++j)
-      if (j == jl) {
-        plp = pl[j];
-        pvl = pv[j];
-      }
-    if (pvl == 0.0) continue;
-    ud -= plp * a.plu[__ldg(R.pt_ue + e)];
-  }
-  if (fabs(ud) <= kEps) ud = fabs(de) > kEps ? de : 1.0;
-  a.pdiag[i] = ud;
-  a.plu[dp] = 0.0;
-  for (int k = dp + 1; k < b1; ++k) {
-    const double v = __ldg(a.pval + k);
-    a.plu[k] = v == 0.0 ? 0.0 : v;
-  }
-}
-
-// Both ILU0 rows of a row of at most 32 blocks (a perforated cell's row with its well's fill) by
-// one warp, from the update lists: lane j holds entry b0 + j of the row in registers, so the
-// sequential walk over the row's lower entries costs shuffles instead of global round trips.
-// Every element gets the operations of block_ilu_row / pressure_ilu_row in their order:
-//  - block: for each present lower entry kp in turn, every lane forms L_ik = lu_kp Dinv_col[kp]
-//    (both shuffled from lane kp); lane e takes the e-th pair (up, ip) of kp's list and forms
-//    L_ik U_up; lane ip - b0 subtracts it from its block (each pair updates a different block);
-//    lane kp's block becomes L_ik;
-//  - pressure: each lower entry in turn, its terms plu[lp] U(col[lp], c) formed by one lane each
-//    and summed in list order; then the diagonal; the upper entries each by their own lane.
-// s_src and s_pl are this warp's 32-entry shared-memory scratch.
-__device__ void ilu_rows_lanes(int i, const FacArgs& a, int* s_src, double* s_pl) {
-  constexpr unsigned kAll = 0xffffffffu;
-  const int lane = threadIdx.x & 31;
-  const int* rp = a.L.rp;
-  const int* col = a.L.col;
-  const FacRecipes& R = a.R;
-  const int b0 = rp[i], dp = a.L.diag[i], b1 = rp[i + 1];
-  const int len = b1 - b0, nl = dp - b0;
-  const int k = b0 + lane;
-  const bool own = lane < len;
-  const bool m = own && a.mask[k];
-  double blk[9], dv[9];
-#pragma unroll
-  for (int e = 0; e < 9; ++e) blk[e] = m ? a.val[size_t(k) * 9 + e] : 0.0;
-  const int ck = own ? col[k] : 0;
-#pragma unroll
-  for (int e = 0; e < 9; ++e) dv[e] = lane < nl ? a.dinv[size_t(ck) * 9 + e] : 0.0;
-  const unsigned present = __ballot_sync(kAll, m);
-  for (int kp = 0; kp < nl; ++kp) {
-    if (!((present >> kp) & 1u)) continue;  // uniform over the warp
-    double lk[9], dk[9], lik[9];
-#pragma unroll
-    for (int e = 0; e < 9; ++e) {
-      lk[e] = __shfl_sync(kAll, blk[e], kp);
-      dk[e] = __shfl_sync(kAll, dv[e], kp);
-    }
-    mat3_mul(lk, dk, lik);
-    const int e0 = R.tri_ptr[b0 + kp], np = R.tri_ptr[b0 + kp + 1] - e0;
-    int tgt = -1;
-    double prod[9];
-#pragma unroll
-    for (int e = 0; e < 9; ++e) prod[e] = 0.0;
-    if (lane < np) {
-      const int up = R.tri_up[e0 + lane], ip = R.tri_ip[e0 + lane];
-      if (a.mask[up] && a.mask[ip]) {
-        double u[9];
-#pragma unroll
-        for (int e = 0; e < 9; ++e) u[e] = a.lu[size_t(up) * 9 + e];
-        mat3_mul(lik, u, prod);
-        tgt = ip - b0;
-      }
-    }
-    s_src[lane] = -1;
-    __syncwarp();
-    if (tgt >= 0) s_src[tgt] = lane;
-    __syncwarp();
-    const int src = s_src[lane];
-#pragma unroll
-    for (int e = 0; e < 9; ++e) {
-      const double v = __shfl_sync(kAll, prod[e], src >= 0 ? src : lane);
-      if (src >= 0) blk[e] -= v;
-    }
-    if (lane == kp) {
-#pragma unroll
-      for (int e = 0; e < 9; ++e) blk[e] = lik[e];
-    }
-  }
-  if (lane == nl) mat3_inverse_or_diag(blk, a.dinv + size_t(i) * 9);
-  if (own) {
-#pragma unroll
-    for (int e = 0; e < 9; ++e) a.lu[size_t(k) * 9 + e] = blk[e];
-  }
-  // pressure ILU0
-  const double pv = own ? a.pval[k] : 0.0;
-  const double pdg = lane < nl ? a.pdiag[ck] : 0.0;
-  const unsigned pnz = __ballot_sync(kAll, own && pv != 0.0);
-  double pl = 0.0;
-  // s0 minus the terms of entry kk in list order (entries whose lp has a zero value skipped)
-  auto terms = [&](int kk, double s0) {
-    const int e0 = R.pt_ptr[kk], nt = R.pt_ptr[kk + 1] - e0;
-    int lpl = lane;
-    double ue = 0.0;
-    if (lane < nt) {
-      lpl = R.pt_lp[e0 + lane] - b0;
-      ue = a.plu[R.pt_ue[e0 + lane]];
-    }
-    const double plp = __shfl_sync(kAll, pl, lpl);
-    const bool valid = lane < nt && ((pnz >> lpl) & 1u);
-    const double term = valid ? plp * ue : 0.0;
-    double s = s0;
-    for (int q = 0; q < nt; ++q) {
-      const double tq = __shfl_sync(kAll, term, q);
-      if (__shfl_sync(kAll, int(valid), q)) s -= tq;
-    }
-    return s;
-  };
-  for (int kp = 0; kp < nl; ++kp) {
-    if (!((pnz >> kp) & 1u)) continue;  // plu stays 0
-    const double s = terms(b0 + kp, __shfl_sync(kAll, pv, kp));
-    const double d = __shfl_sync(kAll, pdg, kp);
-    if (lane == kp) pl = fabs(d) > kEps ? s / d : 0.0;
-  }
-  {
-    const double de = __shfl_sync(kAll, pv, nl);
-    double ud = terms(dp, de);
-    if (fabs(ud) <= kEps) ud = fabs(de) > kEps ? de : 1.0;
-    if (lane == 0) a.pdiag[i] = ud;
-  }
-  // upper entries: each lane its own, reading the row's lower values from shared memory
-  s_pl[lane] = pl;
-  __syncwarp();
-  if (own && lane > nl && pv != 0.0) {
-    double s = pv;
-    for (int e = R.pt_ptr[k]; e < R.pt_ptr[k + 1]; ++e) {
-      const int lpl = R.pt_lp[e] - b0;
-      if (!((pnz >> lpl) & 1u)) continue;
-      s -= s_pl[lpl] * a.plu[R.pt_ue[e]];
-    }
-    pl = s;
-  }
-  if (own) a.plu[k] = lane == nl ? 0.0 : pl;
-  __syncwarp();
-}
-
-// One factorisation on one thread-block cluster: each level's short rows spread over all CTAs'
-// threads, the rows with a well's fill over their warps, one cluster barrier per level.
+// The searching form of the factorisation on one thread-block cluster: each level's short rows spread
+// over all CTAs' threads, the rows with a well's fill over their warps, one cluster barrier per
+// level.  It runs where RESSIM_FACTOR_RECIPES=0 asks for it and is what the tests compare the
+// factorisation from the plan (rf_factor.cu) with.
 __global__ void __launch_bounds__(kFBlock, 1) k_factor_cluster(const __grid_constant__ FacArgs a) {
   __shared__ int s_ptr[kSmemLevels];
-  __shared__ int s_src[kFBlock];
-  __shared__ double s_pl[kFBlock];
   const LevelSched& L = a.L;
   const int* lp = stage_levels(L, s_ptr);
   const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
-  const int warp = tid >> 5, nwarps = nth >> 5, lw = threadIdx.x >> 5;
-  for (int l = 0; l < L.n_levels; ++l) {
-    for (int q = lp[l] + tid; q < lp[l + 1]; q += nth) {
-      const int r = L.lvl_rows[q];
-      if (L.rp[r + 1] - L.rp[r] > kLongRowBlocks) continue;  // a warp takes it below
-      if (a.R.tri_ptr) {
-        if (a.R.simple[r])
-          ilu_row_simple(r, a);
-        else
-          ilu_row_recipe(r, a);
-      } else {
-        block_ilu_row(r, L.rp, L.col, L.diag, a.val, a.mask, a.lu, a.dinv);
-        pressure_ilu_row(r, L.rp, L.col, L.diag, a.pval, a.plu, a.pdiag);
-      }
-    }
-    __syncwarp();
-    for (int q = L.long_ptr[l] + warp; q < L.long_ptr[l + 1]; q += nwarps) {
-      const int r = L.long_rows[q];
-      if (a.R.tri_ptr && L.rp[r + 1] - L.rp[r] <= 32)
-        ilu_rows_lanes(r, a, s_src + 32 * lw, s_pl + 32 * lw);
-      else
-        ilu_rows_warp(r, L.rp, L.col, L.diag, a.val, a.mask, a.lu, a.dinv, a.pval, a.plu, a.pdiag);
-    }
-    cluster_barrier();
-  }
-}
-
-// The same factorisation for many contexts in one launch (the ensemble's batched stepping, and
-// the level-order path with one item): thread block b factors item b's matrices alone, level by
-// level, with block barriers.  Every row gets the operations of k_factor_cluster, so the factors
-// do not depend on the launch.
-struct FacBatch {
-  int count;
-  FacArgs item[kBatchItems];
-};
-__global__ void __launch_bounds__(kFBlock, 1) k_factor_batch(const __grid_constant__ FacBatch b) {
-  if (blockIdx.x >= unsigned(b.count)) return;  // uniform over the block
-  const FacArgs& a = b.item[blockIdx.x];
-  const LevelSched& L = a.L;
-  __shared__ int s_ptr[kSmemLevels];
-  const int* lp = stage_levels(L, s_ptr);
-  __shared__ int s_src[kFBlock];
-  __shared__ double s_pl[kFBlock];
-  const int tid = threadIdx.x, nth = blockDim.x;
   const int warp = tid >> 5, nwarps = nth >> 5;
   for (int l = 0; l < L.n_levels; ++l) {
     for (int q = lp[l] + tid; q < lp[l + 1]; q += nth) {
       const int r = L.lvl_rows[q];
       if (L.rp[r + 1] - L.rp[r] > kLongRowBlocks) continue;  // a warp takes it below
-      if (a.R.tri_ptr) {
-        if (a.R.simple[r])
-          ilu_row_simple(r, a);
-        else
-          ilu_row_recipe(r, a);
-      } else {
-        block_ilu_row(r, L.rp, L.col, L.diag, a.val, a.mask, a.lu, a.dinv);
-        pressure_ilu_row(r, L.rp, L.col, L.diag, a.pval, a.plu, a.pdiag);
-      }
+      block_ilu_row(r, L.rp, L.col, L.diag, a.val, a.mask, a.lu, a.dinv);
+      pressure_ilu_row(r, L.rp, L.col, L.diag, a.pval, a.plu, a.pdiag);
     }
     __syncwarp();
-    for (int q = L.long_ptr[l] + warp; q < L.long_ptr[l + 1]; q += nwarps) {
-      const int r = L.long_rows[q];
-      if (a.R.tri_ptr && L.rp[r + 1] - L.rp[r] <= 32)
-        ilu_rows_lanes(r, a, s_src + 32 * warp, s_pl + 32 * warp);
-      else
-        ilu_rows_warp(r, L.rp, L.col, L.diag, a.val, a.mask, a.lu, a.dinv, a.pval, a.plu, a.pdiag);
-    }
-    __syncthreads();
+    for (int q = L.long_ptr[l] + warp; q < L.long_ptr[l + 1]; q += nwarps)
+      ilu_rows_warp(L.long_rows[q], L.rp, L.col, L.diag, a.val, a.mask, a.lu, a.dinv, a.pval, a.plu, a.pdiag);
+    cluster_barrier();
   }
-}
-static_assert(sizeof(FacArgs) <= kBatchArgBytes, "factorisation arguments must fit a batch item");
-
-bool launch_factor_batch(const BatchItem* const* items, int count, cudaStream_t stream) {
-  FacBatch b;
-  b.count = count;
-  for (int i = 0; i < count; ++i) std::memcpy(&b.item[i], items[i]->args, sizeof(FacArgs));
-  void* args[] = {&b};
-  return cudaLaunchKernel((const void*)k_factor_batch, dim3(count), dim3(kFBlock), args, 0, stream) == cudaSuccess;
 }
 
 // ============================================================================================
@@ -2242,26 +1832,10 @@ static void cpr_build(Ctx& c) {
     k_pressure_matrix<<<blocks_for(n), kBlock, 0, c.stream>>>(n, c.d_row_ptr.p, c.d_val.p, c.d_cpr_w.p, c.d_pval.p);
   }
   c.launches += 2;
-  LevelSched L = level_sched(c);
-  const double* val = c.d_val.p;
-  const unsigned char* mask = c.d_bmask.p;
-  double* lu = c.d_lu.p;
-  double* dinv = c.d_dinv.p;
-  const double* pval = c.d_pval.p;
-  double* plu = c.d_plu.p;
-  double* pdiag = c.d_pdiag.p;
-  FacRecipes rec{c.d_tri_ptr.p, c.d_tri_up.p, c.d_tri_ip.p, c.d_pt_ptr.p, c.d_pt_lp.p, c.d_pt_ue.p, c.d_fac_simple.p};
-  const FacArgs fa{L, val, mask, lu, dinv, pval, plu, pdiag, rec};
-  if (c.batched && fiber_file(kBatchFactor, 0, &fa, sizeof(fa), kFBlock, 0)) {
-    // filed with the group's batched launch
-  } else if (level_solver_active(c)) {
-    // the level-order path: one thread block with the update lists
-    FacBatch fb;
-    fb.count = 1;
-    fb.item[0] = fa;
-    k_factor_batch<<<1, kFBlock, 0, c.stream>>>(fb);
-    c.launches++;
+  if (c.fac.built) {
+    factor_levels(c);
   } else {
+    const FacArgs fa{level_sched(c), c.d_val.p, c.d_bmask.p, c.d_lu.p, c.d_dinv.p, c.d_pval.p, c.d_plu.p, c.d_pdiag.p};
     void* args[] = {(void*)&fa};
     cluster_launch(c, (const void*)k_factor_cluster, kFBlock, args);
   }
@@ -2769,76 +2343,6 @@ LinResult linear_solve_full(Ctx& c, std::vector<double>& h_dx_tail) {
 
 // ---- one-time setup ----
 // Update lists of the factorisation (FacRecipes) for the current pattern.
-void build_factor_recipes(Ctx& c) {
-  // RESSIM_FACTOR_RECIPES=0 (read when a context is set up) keeps the searching forms of the
-  // factorisation instead; the two give identical factors, which the tests check through it
-  const char* env = std::getenv("RESSIM_FACTOR_RECIPES");
-  if (env && std::strcmp(env, "0") == 0) return;
-  const int n = c.n, nnzb = c.nnzb;
-  std::vector<int> tri_ptr(nnzb + 1, 0), tri_up, tri_ip, pt_ptr(nnzb + 1, 0), pt_lp, pt_ue;
-  auto find_in_row_upper = [&](int row, int colj) -> int {
-    const int lo = c.h_diag[row] + 1, hi = c.h_row_ptr[row + 1];
-    auto b = c.h_col.begin() + lo, e = c.h_col.begin() + hi;
-    auto it = std::lower_bound(b, e, colj);
-    return (it != e && *it == colj) ? int(it - c.h_col.begin()) : -1;
-  };
-  for (int i = 0; i < n; ++i) {
-    const int b0 = c.h_row_ptr[i], dp = c.h_diag[i], b1 = c.h_row_ptr[i + 1];
-    for (int k = b0; k < b1; ++k) {
-      if (k < dp) {  // block ILU: U-row of col[k] against row i's later entries
-        const int kr = c.h_col[k];
-        int ip = k + 1;
-        for (int up = c.h_diag[kr] + 1; up < c.h_row_ptr[kr + 1]; ++up) {
-          const int j = c.h_col[up];
-          while (ip < b1 && c.h_col[ip] < j) ++ip;
-          if (ip >= b1) break;
-          if (c.h_col[ip] != j) continue;
-          tri_up.push_back(up);
-          tri_ip.push_back(ip);
-        }
-      }
-      tri_ptr[k + 1] = int(tri_up.size());
-      // pressure ILU: earlier lower entries lp whose row holds col[k] above its diagonal
-      const int lp_end = k < dp ? k : dp;
-      for (int lp = b0; lp < lp_end; ++lp) {
-        const int ue = find_in_row_upper(c.h_col[lp], c.h_col[k]);
-        if (ue < 0) continue;
-        pt_lp.push_back(lp);
-        pt_ue.push_back(ue);
-      }
-      pt_ptr[k + 1] = int(pt_lp.size());
-    }
-  }
-  auto up = [](DBuf<int>& b, const std::vector<int>& h) {
-    b.free();
-    b.alloc(h.size());
-    if (!h.empty()) RF_CUDA(cudaMemcpy(b.p, h.data(), sizeof(int) * h.size(), cudaMemcpyHostToDevice));
-  };
-  // rows of the simple shape (ilu_row_simple): few lower entries, each updating only the
-  // diagonal, and pressure terms only on the diagonal
-  std::vector<unsigned char> simple(n, 0);
-  for (int i = 0; i < n; ++i) {
-    const int b0 = c.h_row_ptr[i], dp = c.h_diag[i], b1 = c.h_row_ptr[i + 1];
-    bool ok = dp - b0 <= 4 && b1 - b0 <= kLongRowBlocks;  // kSimpleLower
-    for (int k = b0; ok && k < dp; ++k) {
-      const int cnt = tri_ptr[k + 1] - tri_ptr[k];
-      if (cnt > 1 || (cnt == 1 && tri_ip[tri_ptr[k]] != dp)) ok = false;
-    }
-    for (int k = b0; ok && k < b1; ++k)
-      if (k != dp && pt_ptr[k + 1] != pt_ptr[k]) ok = false;
-    simple[i] = ok ? 1 : 0;
-  }
-  c.d_fac_simple.free();
-  c.d_fac_simple.alloc(size_t(n));
-  RF_CUDA(cudaMemcpy(c.d_fac_simple.p, simple.data(), size_t(n), cudaMemcpyHostToDevice));
-  up(c.d_tri_ptr, tri_ptr);
-  up(c.d_tri_up, tri_up);
-  up(c.d_tri_ip, tri_ip);
-  up(c.d_pt_ptr, pt_ptr);
-  up(c.d_pt_lp, pt_lp);
-  up(c.d_pt_ue, pt_ue);
-}
-
 void build_levels(Ctx& c) {
   const int n = c.n;
   std::vector<int> lvl(n, 0);
@@ -3125,7 +2629,10 @@ void setup_linear_workspace(Ctx& c) {
   set_cluster_size(c, auto_cluster_size(c));
   build_level_plan(c);
   build_pencil_plan(c);
-  build_factor_recipes(c);
+  // RESSIM_FACTOR_RECIPES=0 (read when a context is set up) keeps the searching form of the
+  // factorisation; the two give identical factors, which the tests check through it
+  const char* env = std::getenv("RESSIM_FACTOR_RECIPES");
+  if (!env || std::strcmp(env, "0") != 0) build_factor_plan(c);
   const int nt = 1 + c.topo.max_perfs_per_well;
   const size_t smem = sizeof(double) * (2 * size_t(nt) * nt + 2 * nt);
   if (smem > 48 * 1024) raise_dynamic_smem((const void*)k_schur, smem);

@@ -95,6 +95,12 @@ void level_pack(Ctx& c);
 void launch_bicgstab_level(Ctx& c, const double* rhs, double* x);
 void launch_block_sweep_level(Ctx& c, const double* cr, double* x, const void* lu, const void* dinv);
 
+// The ILU0 factorisations of d_val and d_pval (rf_factor.cu): plan of the current pattern, once per
+// topology, and the launches.
+void build_factor_plan(Ctx& c);
+void free_factor_plan(Ctx& c);
+void factor_levels(Ctx& c);
+
 // Largest deck whose pressure stage is the dense inverse of its matrix.
 constexpr int kDenseCoarseCells = 299;
 
