@@ -1,9 +1,10 @@
 // rf_blackoil.cu — device kernels of the three-phase black-oil mode.  They mirror the two-phase
 // kernels of rf_assembly.cu / rf_state.cu with the black-oil physics of rf_blackoil.cuh:
 //
-// k_cells3      one thread per cell: accumulation (Dual<3>) and the six face fluxes (Dual<6> over
-//               both neighbours' [p, sw, hc]), each in its cell's regime, written straight into
-//               the cell's block row in the reference's triplet order (fim/assembly_ad.rs:782-983)
+// k_terms3      accumulation (Dual<3>) and the fluxes of three faces per cell (Dual<6> over both
+//               neighbours' [p, sw, hc]), each in its cell's regime
+// k_rows3       the cells' block rows from those terms, in the reference's triplet order
+//               (fim/assembly_ad.rs:782-983)
 // k_perfs3      perforation source terms and rows (fim/assembly_ad.rs:239-577), gas injection
 // k_wells3      control rows (fim/wells_ad.rs:345-378)
 // k_norms3      scaled residual maxima and CNV/MB partials with Bo at the simulator's Rs and Bg
@@ -21,20 +22,113 @@
 
 namespace rf {
 
-__global__ void __launch_bounds__(128) k_cells3(const __grid_constant__ Fluid f, int nx, int ny, int nz, double dt,
-                                                 const double* __restrict__ pv, const double* __restrict__ tx,
-                                                 const double* __restrict__ ty, const double* __restrict__ tz,
-                                                 const double* __restrict__ depth, const int* __restrict__ reg,
-                                                 const double* __restrict__ p, const double* __restrict__ sw,
-                                                 const double* __restrict__ hc, const double* __restrict__ pp,
-                                                 const double* __restrict__ psw, const double* __restrict__ phc,
-                                                 const int* __restrict__ row_ptr, const int* __restrict__ stencil,
-                                                 double* __restrict__ res, double* __restrict__ val,
-                                                 const double* __restrict__ base_rs) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nx * ny * nz) return;
-  cell_row3(f, nx, ny, nz, i, dt, pv, tx, ty, tz, depth, reg, p, sw, hc, pp, psw, phc, row_ptr, stencil, res, val,
-            base_rs);
+// A warp evaluates one kind of term for 32 cells, so that its lanes take one path but for the
+// cells' own regimes and upwind sides, and a small deck's chain is one term long: warps 0-2 the flux
+// values of the x+, y+ and z+ faces, 3-5 their derivatives, 6 the inventory change, 7 its
+// derivatives.  terms: [3 faces][kFaceTerms][n], then [kCellTerms][n].
+// What bounds it: a small deck, one term's chain of FP64 operations and divisions (the Dual<6> flux);
+// a large one, the same at the occupancy 255 registers allow.  A thread per cell that evaluated
+// all six faces, each face of the deck twice, took 455 us at 300 cells and 1,239 us at 72,000;
+// the two kernels take 49 + 5 us and 603 + 71 us.
+constexpr int kTermWarps = 8;
+__global__ void __launch_bounds__(32 * kTermWarps) k_terms3(const __grid_constant__ Fluid f,
+                                                            const __grid_constant__ CellFields3 c,
+                                                            double* __restrict__ terms) {
+  const int n = c.nx * c.ny * c.nz, i = 32 * blockIdx.x + (threadIdx.x & 31), role = threadIdx.x >> 5;
+  if (i >= n) return;
+  const size_t N = size_t(n);
+  if (role < 6) {
+    const int dir = role % 3;
+    int hi;
+    const double t = face3(c, i, dir, hi);
+    if (!(t > 0.0)) return;  // k_rows3 does not read them
+    double* out = terms + dir * kFaceTerms * N + i;
+    if (role < 3) {
+      double fv[kFaceValues];
+      face_values3(f, c, i, hi, t, fv);
+#pragma unroll
+      for (int e = 0; e < kFaceValues; ++e) out[e * N] = fv[e];
+    } else {
+      double d[kFaceDerivs];
+      face_derivs3(f, c, i, hi, t, d);
+#pragma unroll
+      for (int e = 0; e < kFaceDerivs; ++e) out[(kFaceValues + e) * N] = d[e];
+    }
+    return;
+  }
+  double* out = terms + 3 * kFaceTerms * N + i;
+  if (role == 6) {
+    double r[kCellValues];
+    cell_values3(f, c, i, r);
+#pragma unroll
+    for (int e = 0; e < kCellValues; ++e) out[e * N] = r[e];
+  } else {
+    double d[kCellDerivs];
+    cell_derivs3(f, c, i, d);
+#pragma unroll
+    for (int e = 0; e < kCellDerivs; ++e) out[(kCellValues + e) * N] = d[e];
+  }
+}
+
+// Residual and Jacobian rows from the terms, eight lanes per cell: lanes 0-5 the neighbours' blocks
+// (z-, y-, x-, x+, y+, z+), lane 6 the residual and the diagonal block, summed in that order, lane 7
+// zeros in the row's blocks of a well's fill.
+__global__ void __launch_bounds__(kBlock) k_rows3(const __grid_constant__ CellFields3 c, double dt,
+                                                  const double* __restrict__ terms, const int* __restrict__ row_ptr,
+                                                  const int* __restrict__ stencil, double* __restrict__ res,
+                                                  double* __restrict__ val) {
+  const int n = c.nx * c.ny * c.nz, lane = threadIdx.x & 7;
+  const long long at = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 3;
+  if (at >= n) return;
+  const int i = int(at), nxy = c.nx * c.ny;
+  const size_t N = size_t(n);
+  const int* st = stencil + 7 * size_t(i);
+  const int pos[3] = {i % c.nx, (i / c.nx) % c.ny, i / nxy}, step[3] = {1, c.nx, nxy};
+  // the face towards lower (up false) or higher indices along dir, if there is one: its terms
+  auto face = [&](int dir, bool up) -> const double* {
+    if (!up && pos[dir] == 0) return nullptr;
+    const int lo = up ? i : i - step[dir];
+    int hi;
+    return face3(c, lo, dir, hi) > 0.0 ? terms + dir * kFaceTerms * N + lo : nullptr;
+  };
+  if (lane < 6) {
+    const bool up = lane >= 3;
+    const int dir = up ? lane - 3 : 2 - lane;
+    const int k = st[dir == 0 ? (up ? kXp : kXm) : dir == 1 ? (up ? kYp : kYm) : (up ? kZp : kZm)];
+    if (k < 0) return;
+    const double* t = face(dir, up);
+#pragma unroll
+    for (int e = 0; e < 9; ++e) val[size_t(k) * 9 + e] = t ? face_off3(t, N, dt, up, e) : 0.0;
+  } else if (lane == 6) {
+    const double* own = terms + 3 * kFaceTerms * N + i;
+    double r[3], diag[9];
+#pragma unroll
+    for (int e = 0; e < 3; ++e) r[e] = own[e * N];
+#pragma unroll
+    for (int e = 0; e < 9; ++e) diag[e] = own[(kCellValues + e) * N];
+#pragma unroll
+    for (int s = 0; s < 6; ++s) {
+      const double* t = face(s < 3 ? 2 - s : s - 3, s >= 3);
+      if (!t) continue;
+      if (s < 3)
+        face_add3<false>(t, N, dt, r, diag);
+      else
+        face_add3<true>(t, N, dt, r, diag);
+    }
+#pragma unroll
+    for (int e = 0; e < 3; ++e) res[3 * size_t(i) + e] = r[e];
+#pragma unroll
+    for (int e = 0; e < 9; ++e) val[size_t(st[kDiag]) * 9 + e] = diag[e];
+  } else {
+    for (int k = row_ptr[i]; k < row_ptr[i + 1]; ++k) {
+      bool stencil_block = false;
+#pragma unroll
+      for (int s = 0; s < 7; ++s) stencil_block = stencil_block || st[s] == k;
+      if (stencil_block) continue;
+#pragma unroll
+      for (int e = 0; e < 9; ++e) val[size_t(k) * 9 + e] = 0.0;
+    }
+  }
 }
 
 __global__ void k_perfs3(const __grid_constant__ Fluid f, int n_wells, int n_perfs, double dt, const int* __restrict__ perf_cell,
@@ -46,10 +140,11 @@ __global__ void k_perfs3(const __grid_constant__ Fluid f, int n_wells, int n_per
                          double* __restrict__ res, double* __restrict__ val, double* __restrict__ res_tail,
                          double* __restrict__ jrw, double* __restrict__ jwr_perf, double* __restrict__ jww_perf_bhp,
                          const double* __restrict__ base_rs) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  // 32 perforations per block, a warp for each of the four evaluations
+  const int k = 32 * blockIdx.x + (threadIdx.x & 31);
   if (k >= n_perfs) return;
   perf_row3(f, n_wells, k, dt, perf_cell, perf_inj, perf_well, perf_has_wi, perf_wi, perf_head, reg, p, sw, hc, bhp,
-            q, diag_pos, res, val, res_tail, jrw, jwr_perf, jww_perf_bhp, base_rs);
+            q, diag_pos, res, val, res_tail, jrw, jwr_perf, jww_perf_bhp, base_rs, int(threadIdx.x) >> 5);
 }
 
 __global__ void k_wells3(const __grid_constant__ Fluid f, int n_wells, const WellControlH* __restrict__ ctrl, const int* __restrict__ well_ptr,
@@ -244,13 +339,17 @@ static int red_blocks3(const Ctx& c) {
 }
 
 void launch_assembly3(Ctx& c, double dt) {
-  k_cells3<<<blocks_for(c.n, 128), 128, 0, c.stream>>>(c.fluid, c.nx, c.ny, c.nz, dt, c.d_pv.p, c.d_tx.p, c.d_ty.p,
-                                                        c.d_tz.p, c.d_depth.p, c.d_reg.p, c.d_p.p, c.d_sw.p, c.d_hc.p,
-                                                        c.d_pp.p, c.d_psw.p, c.d_phc.p, c.d_row_ptr.p, c.d_stencil.p,
-                                                        c.d_res.p, c.d_val.p, c.d_rs.p);
-  c.launches++;
+  const CellFields3 cf{c.nx, c.ny, c.nz, c.d_pv.p, c.d_tx.p, c.d_ty.p, c.d_tz.p, c.d_depth.p, c.d_reg.p,
+                       c.d_p.p, c.d_sw.p, c.d_hc.p, c.d_pp.p, c.d_psw.p, c.d_phc.p, c.d_rs.p};
+  // the terms lie in the FGMRES basis, which holds nothing between two linear solves
+  static_assert(3 * kFaceTerms + kCellTerms <= 3 * (Ctx::kRestart + 1), "the basis must hold the terms");
+  double* terms = c.d_V.p;
+  k_terms3<<<blocks_for(c.n, 32), 32 * kTermWarps, 0, c.stream>>>(c.fluid, cf, terms);
+  k_rows3<<<int((8ll * c.n + kBlock - 1) / kBlock), kBlock, 0, c.stream>>>(cf, dt, terms, c.d_row_ptr.p,
+                                                                          c.d_stencil.p, c.d_res.p, c.d_val.p);
+  c.launches += 2;
   if (c.topo.n_perfs > 0) {
-    k_perfs3<<<blocks_for(c.topo.n_perfs, 64), 64, 0, c.stream>>>(
+    k_perfs3<<<blocks_for(c.topo.n_perfs, 32), 32 * kPerfParts, 0, c.stream>>>(
         c.fluid, c.topo.n_wells, c.topo.n_perfs, dt, c.d_perf_cell.p, c.d_perf_inj.p, c.d_perf_well.p,
         c.d_perf_has_wi.p, c.d_perf_wi.p, c.d_perf_head.p, c.d_reg.p, c.d_p.p, c.d_sw.p, c.d_hc.p, c.d_bhp.p, c.d_q.p,
         c.d_diag.p, c.d_res.p, c.d_val.p, c.d_res_tail.p, c.d_jrw.p, c.d_jwr_perf.p, c.d_jww_perf_bhp.p, c.d_rs.p);

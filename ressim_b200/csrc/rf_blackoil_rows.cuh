@@ -1,7 +1,9 @@
 // rf_blackoil_rows.cuh — one cell's, one perforation's and one well's residual and Jacobian rows
-// in the three-phase black-oil mode, as __host__ __device__ functions: the kernels k_cells3,
-// k_perfs3 and k_wells3 run them per thread, and a host build runs the same code on the CPU
-// against the oracle's assembly.  Contributions follow the reference's triplet order
+// in the three-phase black-oil mode, as __host__ __device__ functions: the kernels k_terms3,
+// k_rows3, k_perfs3 and k_wells3 run them, and a host build runs the same code on the CPU
+// against the oracle's assembly.  cell_row3 is the host build's whole row;
+// the device evaluates the terms it is made of in one kernel and adds them up in a second one.
+// Contributions follow the reference's triplet order
 // (fim/assembly_ad.rs:782-983): accumulation, then faces z-, y-, x-, x+, y+, z+, then wells;
 // Jacobian entries with |v| <= 1e-14 are dropped before they are added.
 #pragma once
@@ -12,36 +14,84 @@ namespace rf {
 
 RF_HD double filt3(double v) { return fabs(v) > 1e-14 ? v : 0.0; }
 
-template <int DIR_SIGN>
-RF_HD_CALL void face_contrib3(const Fluid& f, double trans, double dt, double depth_lo,
-                         double depth_hi, int reg_lo, double p_lo, double sw_lo, double hc_lo,
-                         int reg_hi, double p_hi, double sw_hi, double hc_hi, double r[3],
-                         double diag[9], double* off, double base_lo, double base_hi) {
-  // lower-index cell = "i" (slots 0-2), higher = "j" (slots 3-5); DIR_SIGN +1: this cell is i
-  double fv[3];
-  face_flux3<double>(f, trans, depth_lo, depth_hi, reg_lo, p_lo, sw_lo, hc_lo, reg_hi, p_hi, sw_hi, hc_hi, fv,
-                     base_lo, base_hi);
+// The terms a cell's row is made of.  A face's are evaluated once, for both of its cells: the three
+// component fluxes (kFaceValues) and their derivatives by the lower-index cell's [p, sw, hc], then
+// the higher's (kFaceDerivs); the cell's own are the inventory change and the inventory's
+// derivatives.  Device code keeps them in arrays of n cells, [term][cell].
+constexpr int kFaceValues = 3, kFaceDerivs = 18, kFaceTerms = kFaceValues + kFaceDerivs;
+constexpr int kCellValues = 3, kCellDerivs = 9, kCellTerms = kCellValues + kCellDerivs;
+
+// What the row functions read of the deck and its state.
+struct CellFields3 {
+  int nx, ny, nz;
+  const double *pv, *tx, *ty, *tz, *depth;
+  const int* reg;
+  const double *p, *sw, *hc, *pp, *psw, *phc, *base_rs;
+};
+// the DRSDT0 Rs cap of a cell: the simulator's Rs at the substep start
+RF_HD double base3(const Fluid& f, const CellFields3& c, int i) { return f.drsdt0 ? c.base_rs[i] : 0.0; }
+
+// The face from cell i to its next one along `dir` (0 x, 1 y, 2 z): transmissibility (0: none), other cell.
+RF_HD double face3(const CellFields3& c, int i, int dir, int& hi) {
+  const int nxy = c.nx * c.ny, at = dir == 0 ? i % c.nx : dir == 1 ? (i / c.nx) % c.ny : i / nxy;
+  hi = i + (dir == 0 ? 1 : dir == 1 ? c.nx : nxy);
+  if (at + 1 >= (dir == 0 ? c.nx : dir == 1 ? c.ny : c.nz)) return 0.0;
+  return (dir == 0 ? c.tx : dir == 1 ? c.ty : c.tz)[i];
+}
+RF_HD void face_values3(const Fluid& f, const CellFields3& c, int i, int hi, double trans, double fv[3]) {
+  const int nxy = c.nx * c.ny;
+  face_flux3<double>(f, trans, c.depth[i / nxy], c.depth[hi / nxy], c.reg[i], c.p[i], c.sw[i], c.hc[i], c.reg[hi],
+                     c.p[hi], c.sw[hi], c.hc[hi], fv, base3(f, c, i), base3(f, c, hi));
+}
+RF_HD void face_derivs3(const Fluid& f, const CellFields3& c, int i, int hi, double trans, double d[kFaceDerivs]) {
+  const int nxy = c.nx * c.ny;
   Dual<6> fd[3];
-  face_flux3<Dual<6>>(f, trans, depth_lo, depth_hi, reg_lo, dvar<6>(p_lo, 0), dvar<6>(sw_lo, 1), dvar<6>(hc_lo, 2),
-                      reg_hi, dvar<6>(p_hi, 3), dvar<6>(sw_hi, 4), dvar<6>(hc_hi, 5), fd, base_lo, base_hi);
+  face_flux3<Dual<6>>(f, trans, c.depth[i / nxy], c.depth[hi / nxy], c.reg[i], dvar<6>(c.p[i], 0), dvar<6>(c.sw[i], 1),
+                      dvar<6>(c.hc[i], 2), c.reg[hi], dvar<6>(c.p[hi], 3), dvar<6>(c.sw[hi], 4), dvar<6>(c.hc[hi], 5),
+                      fd, base3(f, c, i), base3(f, c, hi));
+#pragma unroll
+  for (int e = 0; e < 3; ++e)
+#pragma unroll
+    for (int v = 0; v < 6; ++v) d[6 * e + v] = fd[e].d[v];
+}
+// accumulation; the previous inventory uses the same (frozen) regime, as the substep's previous
+// state and first iterate are the same classified state
+RF_HD void cell_values3(const Fluid& f, const CellFields3& c, int i, double r[3]) {
+  const double bi = base3(f, c, i);
+  double cur[3], prev[3];
+  inventory3<double>(f, c.pv[i], c.reg[i], c.p[i], c.sw[i], c.hc[i], bi, cur);
+  inventory3<double>(f, c.pv[i], c.reg[i], c.pp[i], c.psw[i], c.phc[i], bi, prev);
+#pragma unroll
+  for (int e = 0; e < 3; ++e) r[e] = 0.0 + (cur[e] - prev[e]);
+}
+RF_HD void cell_derivs3(const Fluid& f, const CellFields3& c, int i, double d[kCellDerivs]) {
+  Dual<3> cd[3];
+  inventory3<Dual<3>>(f, c.pv[i], c.reg[i], dvar<3>(c.p[i], 0), dvar<3>(c.sw[i], 1), dvar<3>(c.hc[i], 2),
+                      base3(f, c, i), cd);
+#pragma unroll
+  for (int e = 0; e < 3; ++e)
+#pragma unroll
+    for (int v = 0; v < 3; ++v) d[3 * e + v] = filt3(cd[e].d[v]);
+}
+// A face's part of a cell's residual and diagonal block; UP: the cell is the face's lower one.
+// Terms lie `stride` apart.
+template <bool UP>
+RF_HD void face_add3(const double* t, size_t stride, double dt, double r[3], double diag[9]) {
 #pragma unroll
   for (int e = 0; e < 3; ++e) {
-    if (DIR_SIGN > 0) {
-      r[e] += fv[e] * dt;
+    const double fv = t[e * stride];
+    r[e] += (UP ? fv : -fv) * dt;
 #pragma unroll
-      for (int v = 0; v < 3; ++v) {
-        diag[3 * e + v] += filt3(fd[e].d[v] * dt);
-        off[3 * e + v] = filt3(fd[e].d[3 + v] * dt);
-      }
-    } else {
-      r[e] += -fv[e] * dt;
-#pragma unroll
-      for (int v = 0; v < 3; ++v) {
-        diag[3 * e + v] += filt3(-fd[e].d[3 + v] * dt);
-        off[3 * e + v] = filt3(-fd[e].d[v] * dt);
-      }
+    for (int v = 0; v < 3; ++v) {
+      const double d = t[(kFaceValues + 6 * e + (UP ? v : 3 + v)) * stride];
+      diag[3 * e + v] += filt3((UP ? d : -d) * dt);
     }
   }
+}
+// Entry k of its block in the column of the face's other cell.
+RF_HD double face_off3(const double* t, size_t stride, double dt, bool up, int k) {
+  const double d = t[(kFaceValues + 6 * (k / 3) + (up ? 3 : 0) + k % 3) * stride];
+  return filt3((up ? d : -d) * dt);
 }
 
 // Residual row and Jacobian block row of cell i (accumulation, then the six faces), written into
@@ -57,94 +107,32 @@ RF_HD void cell_row3(const Fluid& f, int nx, int ny, int nz, int i, double dt,
                      double* __restrict__ res, double* __restrict__ val,
                      const double* __restrict__ base_rs) {
   const int nxy = nx * ny;
-  const int ci = i % nx, cj = (i / nx) % ny, ck = i / nxy;
   for (int k = row_ptr[i]; k < row_ptr[i + 1]; ++k)
 #pragma unroll
     for (int e = 0; e < 9; ++e) val[size_t(k) * 9 + e] = 0.0;
-
-  // accumulation; the previous inventory uses the same (frozen) regime, as the substep's
-  // previous state and first iterate are the same classified state
-  const int ri = reg[i];
-  // the DRSDT0 Rs cap of a cell: the simulator's Rs at the substep start
-  auto base = [&](int c) { return f.drsdt0 ? base_rs[c] : 0.0; };
-  const double bi = base(i);
-  double cur[3], prev[3];
-  inventory3<double>(f, pv[i], ri, p[i], sw[i], hc[i], bi, cur);
-  inventory3<double>(f, pv[i], ri, pp[i], psw[i], phc[i], bi, prev);
-  double r[3] = {0.0 + (cur[0] - prev[0]), 0.0 + (cur[1] - prev[1]), 0.0 + (cur[2] - prev[2])};
-  double diag[9];
-  {
-    Dual<3> cd[3];
-    inventory3<Dual<3>>(f, pv[i], ri, dvar<3>(p[i], 0), dvar<3>(sw[i], 1), dvar<3>(hc[i], 2), bi, cd);
-#pragma unroll
-    for (int e = 0; e < 3; ++e)
-#pragma unroll
-      for (int v = 0; v < 3; ++v) diag[3 * e + v] = filt3(cd[e].d[v]);
-  }
+  const CellFields3 c{nx, ny, nz, pv, tx, ty, tz, depth, reg, p, sw, hc, pp, psw, phc, base_rs};
+  double r[3], diag[9];
+  cell_values3(f, c, i, r);
+  cell_derivs3(f, c, i, diag);
   const int* st = stencil + size_t(i) * 7;
-  double off[9];
-  const double dk = depth[ck];
-  const double pi = p[i], swi = sw[i], hci = hc[i];
-  if (ck > 0) {
-    const int nb = i - nxy;
-    const double t = tz[nb];
-    if (t > 0.0) {
-      face_contrib3<-1>(f, t, dt, depth[ck - 1], dk, reg[nb], p[nb], sw[nb], hc[nb], ri, pi, swi, hci, r, diag, off,
-                        base(nb), bi);
-#pragma unroll
-      for (int e = 0; e < 9; ++e) val[size_t(st[kZm]) * 9 + e] = off[e];
-    }
-  }
-  if (cj > 0) {
-    const int nb = i - nx;
-    const double t = ty[nb];
-    if (t > 0.0) {
-      face_contrib3<-1>(f, t, dt, dk, dk, reg[nb], p[nb], sw[nb], hc[nb], ri, pi, swi, hci, r, diag, off,
-                        base(nb), bi);
-#pragma unroll
-      for (int e = 0; e < 9; ++e) val[size_t(st[kYm]) * 9 + e] = off[e];
-    }
-  }
-  if (ci > 0) {
-    const int nb = i - 1;
-    const double t = tx[nb];
-    if (t > 0.0) {
-      face_contrib3<-1>(f, t, dt, dk, dk, reg[nb], p[nb], sw[nb], hc[nb], ri, pi, swi, hci, r, diag, off,
-                        base(nb), bi);
-#pragma unroll
-      for (int e = 0; e < 9; ++e) val[size_t(st[kXm]) * 9 + e] = off[e];
-    }
-  }
-  if (ci + 1 < nx) {
-    const int nb = i + 1;
-    const double t = tx[i];
-    if (t > 0.0) {
-      face_contrib3<1>(f, t, dt, dk, dk, ri, pi, swi, hci, reg[nb], p[nb], sw[nb], hc[nb], r, diag, off,
-                       bi, base(nb));
-#pragma unroll
-      for (int e = 0; e < 9; ++e) val[size_t(st[kXp]) * 9 + e] = off[e];
-    }
-  }
-  if (cj + 1 < ny) {
-    const int nb = i + nx;
-    const double t = ty[i];
-    if (t > 0.0) {
-      face_contrib3<1>(f, t, dt, dk, dk, ri, pi, swi, hci, reg[nb], p[nb], sw[nb], hc[nb], r, diag, off,
-                       bi, base(nb));
-#pragma unroll
-      for (int e = 0; e < 9; ++e) val[size_t(st[kYp]) * 9 + e] = off[e];
-    }
-  }
-  if (ck + 1 < nz) {
-    const int nb = i + nxy;
-    const double t = tz[i];
-    if (t > 0.0) {
-      face_contrib3<1>(f, t, dt, dk, depth[ck + 1], ri, pi, swi, hci, reg[nb], p[nb], sw[nb], hc[nb], r, diag, off,
-                       bi, base(nb));
-#pragma unroll
-      for (int e = 0; e < 9; ++e) val[size_t(st[kZp]) * 9 + e] = off[e];
-    }
-  }
+  const int at[3] = {i % nx, (i / nx) % ny, i / nxy}, step[3] = {1, nx, nxy};
+  const int lower[3] = {kXm, kYm, kZm}, upper[3] = {kXp, kYp, kZp};
+  auto face = [&](int lo, int dir, bool up) {
+    int hi;
+    const double t = face3(c, lo, dir, hi);
+    if (!(t > 0.0)) return;
+    double terms[kFaceTerms];
+    face_values3(f, c, lo, hi, t, terms);
+    face_derivs3(f, c, lo, hi, t, terms + kFaceValues);
+    if (up)
+      face_add3<true>(terms, 1, dt, r, diag);
+    else
+      face_add3<false>(terms, 1, dt, r, diag);
+    for (int e = 0; e < 9; ++e) val[size_t(st[up ? upper[dir] : lower[dir]]) * 9 + e] = face_off3(terms, 1, dt, up, e);
+  };
+  for (int dir = 2; dir >= 0; --dir)
+    if (at[dir] > 0) face(i - step[dir], dir, false);
+  for (int dir = 0; dir < 3; ++dir) face(i, dir, true);
 #pragma unroll
   for (int e = 0; e < 3; ++e) res[3 * i + e] = r[e];
 #pragma unroll
@@ -152,6 +140,8 @@ RF_HD void cell_row3(const Fluid& f, int nx, int ny, int nz, int i, double dt,
 }
 
 // Perforation k: its source terms in the cell's rows and diagonal block, and its connection row.
+// `part`: kPerfAll, or one of the four independent evaluations (the device gives each a warp).
+constexpr int kPerfAll = -1, kPerfParts = 4;
 RF_HD void perf_row3(const Fluid& f, int n_wells, int k, double dt, const int* __restrict__ perf_cell,
                      const int* __restrict__ perf_inj, const int* __restrict__ perf_well,
                      const int* __restrict__ perf_has_wi, const double* __restrict__ perf_wi,
@@ -160,17 +150,19 @@ RF_HD void perf_row3(const Fluid& f, int n_wells, int k, double dt, const int* _
                      const double* __restrict__ bhp, const double* __restrict__ q, const int* __restrict__ diag_pos,
                      double* __restrict__ res, double* __restrict__ val, double* __restrict__ res_tail,
                      double* __restrict__ jrw, double* __restrict__ jwr_perf, double* __restrict__ jww_perf_bhp,
-                     const double* __restrict__ base_rs) {
+                     const double* __restrict__ base_rs, int part = kPerfAll) {
   const int c = perf_cell[k], w = perf_well[k], rg = reg[c];
   const double bc = f.drsdt0 ? base_rs[c] : 0.0;
   const bool inj = perf_inj[k] != 0;
   const double pc = p[c], swc = sw[c], hcc = hc[c], b = bhp[w], qk = q[k];
-  double coef[3];
-  component_coefficients3<double>(f, inj, rg, pc, swc, hcc, coef, bc);
+  if (part == kPerfAll || part == 0) {
+    double coef[3];
+    component_coefficients3<double>(f, inj, rg, pc, swc, hcc, coef, bc);
 #pragma unroll
-  for (int e = 0; e < 3; ++e) res[3 * c + e] += coef[e] * qk * dt;
-  double* dblk = val + size_t(diag_pos[c]) * 9;
-  {
+    for (int e = 0; e < 3; ++e) res[3 * c + e] += coef[e] * qk * dt;
+  }
+  if (part == kPerfAll || part == 1) {
+    double* dblk = val + size_t(diag_pos[c]) * 9;
     Dual<4> P = dvar<4>(pc, 0), SW = dvar<4>(swc, 1), HC = dvar<4>(hcc, 2), Q = dvar<4>(qk, 3);
     Dual<4> ca[3];
     component_coefficients3<Dual<4>>(f, inj, rg, P, SW, HC, ca, bc);
@@ -182,19 +174,23 @@ RF_HD void perf_row3(const Fluid& f, int n_wells, int k, double dt, const int* _
       jrw[3 * k + e] = filt3(row.d[3] * dt);
     }
   }
-  if (perf_has_wi[k]) {
-    const double conn = connection_rate3<double>(f, perf_wi[k], perf_head[k], inj, rg, pc, swc, hcc, b, bc);
-    res_tail[n_wells + k] = 0.0 + (qk - conn);
-    Dual<4> ca = connection_rate3<Dual<4>>(f, perf_wi[k], perf_head[k], inj, rg, dvar<4>(pc, 0), dvar<4>(swc, 1),
-                                           dvar<4>(hcc, 2), dvar<4>(b, 3), bc);
+  const bool wi = perf_has_wi[k] != 0;
+  if (part == kPerfAll || part == 2) {
+    const double conn = wi ? connection_rate3<double>(f, perf_wi[k], perf_head[k], inj, rg, pc, swc, hcc, b, bc) : 0.0;
+    res_tail[n_wells + k] = wi ? 0.0 + (qk - conn) : 0.0;
+  }
+  if (part == kPerfAll || part == 3) {
+    if (wi) {
+      Dual<4> ca = connection_rate3<Dual<4>>(f, perf_wi[k], perf_head[k], inj, rg, dvar<4>(pc, 0), dvar<4>(swc, 1),
+                                             dvar<4>(hcc, 2), dvar<4>(b, 3), bc);
 #pragma unroll
-    for (int v = 0; v < 3; ++v) jwr_perf[3 * k + v] = filt3(-ca.d[v]);
-    jww_perf_bhp[k] = filt3(-ca.d[3]);
-  } else {
-    res_tail[n_wells + k] = 0.0;
+      for (int v = 0; v < 3; ++v) jwr_perf[3 * k + v] = filt3(-ca.d[v]);
+      jww_perf_bhp[k] = filt3(-ca.d[3]);
+    } else {
 #pragma unroll
-    for (int v = 0; v < 3; ++v) jwr_perf[3 * k + v] = 0.0;
-    jww_perf_bhp[k] = 0.0;
+      for (int v = 0; v < 3; ++v) jwr_perf[3 * k + v] = 0.0;
+      jww_perf_bhp[k] = 0.0;
+    }
   }
 }
 
