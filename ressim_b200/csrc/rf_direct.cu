@@ -12,9 +12,10 @@
 //                     dense column-major matrix and the right-hand side.
 //   k_direct_lu       one thread-block cluster; the columns are dealt round-robin to the CTAs and
 //                     stay in their shared memory (at 512 rows, 32 columns x 512 rows = 128 KB per
-//                     CTA of a 16-CTA cluster).  At step k the owner of column k picks the pivot,
-//                     forms the multipliers and stores them into every CTA's shared memory; after
-//                     one cluster barrier each CTA swaps the two rows and updates its own columns.
+//                     CTA of a 16-CTA cluster).  The owner of column k picks the pivot, forms the
+//                     multipliers and stores them into every CTA's shared memory; after one cluster
+//                     barrier each CTA swaps the two rows and updates its own columns, the owner of
+//                     column k + 1 that one first.
 //                     Partial pivoting takes the first largest |a_ik|; an exactly zero pivot
 //                     column is a failed factorisation.
 //   k_direct_solve    one CTA: x = U^-1 L^-1 P b column by column, factor columns read from L2
@@ -98,91 +99,106 @@ __global__ void k_direct_build_wells(int n_cells, int n_wells, int nf, const int
   }
 }
 
+__device__ __forceinline__ void dir_cluster_arrive() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void dir_cluster_wait() {
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 // LU with partial pivoting, P A = L U, on one cluster of gridDim.x CTAs.  CTA `me` owns the
-// columns j with j % cs == me, in local slot j / cs, column-major in dynamic shared memory.
-// Writes the factors column-major to `lu`, the row permutation to `perm` and status[0] = 1 when
-// every pivot was nonzero (0 otherwise).
-__global__ void __launch_bounds__(kDirThreads) k_direct_lu(int n, const double* __restrict__ a_in,
-                                                            double* __restrict__ lu, int* __restrict__ perm,
-                                                            int* __restrict__ status) {
+// columns j with j % cs == me, in local slot j / cs, column-major in dynamic shared memory; thread t
+// holds row t of them (n <= kDirThreads).
+// What bounds it: the chain of steps.  The owner of column k + 1 updates that column first, picks its
+// pivot and sends the multipliers, and all CTAs update their other columns between arriving at
+// and waiting on the cluster barrier, so a step's chain is one column's update, a reduction, a
+// division and the barrier.  (The update of all columns inside the chain, with an integer division per
+// element, took 5.0 us a step at 325 rows.)
+// Writes the factors to `lu`, the row permutation to `perm` and status[0] = 1 when every pivot was
+// nonzero (0 otherwise).  DENSE: the coarse pressure matrix, row-major and in place (lu == a_in), in
+// nalgebra's operation order (multipliers by the pivot's reciprocal, y = (-p) * c + y with no
+// element left out); else column-major, with the oracle's skip rules.
+template <bool DENSE>
+__global__ void __launch_bounds__(kDirThreads) k_direct_lu(int n, const double* a_in, double* lu,
+                                                            int* __restrict__ perm, int* __restrict__ status) {
   extern __shared__ double dsm[];
   __shared__ int s_piv[2];
   __shared__ int s_perm[kDirectSolveRows];
   __shared__ double s_best[kDirThreads / 32];
   __shared__ int s_arg[kDirThreads / 32];
+  static_assert(kDirectSolveRows <= kDirThreads && kDirThreads / 32 == 16, "a row per thread, sixteen warps");
   const int cs = gridDim.x, t = threadIdx.x, nt = blockDim.x, lane = t & 31, warp = t >> 5;
   const int me = int(dir_cta_rank());
   const int ncl = (n + cs - 1) / cs;
   const int cnt = (n - me + cs - 1) / cs;  // local columns that exist
   double* A = dsm;                // [ncl][n]
   double* lbuf = dsm + size_t(ncl) * n;  // [2][n] multipliers of the current step
-  for (int idx = t; idx < ncl * n; idx += nt) {
-    const int s = idx / n, i = idx % n, j = s * cs + me;
-    A[idx] = j < n ? a_in[size_t(j) * n + i] : 0.0;
+  for (int s = 0; s < ncl; ++s) {
+    const int j = s * cs + me;
+    if (t < n) A[size_t(s) * n + t] = j < n ? (DENSE ? a_in[size_t(t) * n + j] : a_in[size_t(j) * n + t]) : 0.0;
   }
-  if (me == 0)
-    for (int i = t; i < n; i += nt) s_perm[i] = i;
+  if (me == 0 && t < n) s_perm[t] = t;
+  // Pivot and multipliers of column k, to every CTA; by all threads of its owner, v: the column's
+  // value in row t, stored there too.
+  auto publish = [&](int k, double v) {
+    const double* colk = A + size_t(k / cs) * n;
+    const int par = k & 1;
+    // first largest |a_ik| over i >= k: strictly larger replaces, ties keep the smaller row; a NaN
+    // never compares larger, and in row k nothing compares larger than it
+    const bool in = t >= k && t < n, nan = v != v;
+    double best = in ? (nan ? INFINITY : fabs(v)) : -1.0;
+    int arg = in && (!nan || t == k) ? t : -1;
+    auto better = [&](double ob, int oa) {
+      if (oa >= 0 && (arg < 0 || ob > best || (ob == best && oa < arg))) {
+        best = ob;
+        arg = oa;
+      }
+    };
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const double ob = __shfl_xor_sync(0xffffffffu, best, o);
+      const int oa = __shfl_xor_sync(0xffffffffu, arg, o);
+      better(ob, oa);
+    }
+    if (lane == 0) {
+      s_best[warp] = best;
+      s_arg[warp] = arg;
+    }
+    __syncthreads();
+    best = s_best[lane & 15];
+    arg = s_arg[lane & 15];
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) {
+      const double ob = __shfl_xor_sync(0xffffffffu, best, o);
+      const int oa = __shfl_xor_sync(0xffffffffu, arg, o);
+      better(ob, oa);
+    }
+    // an all-zero column fails here, and an all-NaN one that is not DENSE
+    const double piv = arg >= 0 ? colk[arg] : 0.0;
+    const int p = arg >= 0 && (DENSE ? piv != 0.0 : fabs(piv) > 0.0) ? arg : -1;
+    if (p >= 0 && t > k && t < n) {
+      const double w = t == p ? colk[k] : v;
+      const double l = DENSE ? w * (1.0 / piv) : w / piv;
+      for (int r = 0; r < cs; ++r) dir_store_remote(dir_remote(lbuf + size_t(par) * n + t, r), l);
+    }
+    if (t < cs) dir_store_remote(dir_remote(s_piv + par, t), p);
+  };
   // every CTA of the cluster is running before any remote store
   dir_cluster_sync();
+  if (me == 0) publish(0, t < n ? A[t] : 0.0);
+  dir_cluster_arrive();
   for (int k = 0; k < n; ++k) {
-    const int owner = k % cs, par = k & 1;
-    if (me == owner) {
-      const double* colk = A + size_t(k / cs) * n;
-      // first largest |a_ik| over i >= k: strictly larger replaces, ties keep the smaller row
-      double best = -1.0;
-      int arg = -1;
-      for (int i = k + t; i < n; i += nt) {
-        const double v = fabs(colk[i]);
-        if (arg < 0 || v > best) {
-          best = v;
-          arg = i;
-        }
-      }
-      for (int o = 16; o > 0; o >>= 1) {
-        const double ob = __shfl_down_sync(0xffffffffu, best, o);
-        const int oa = __shfl_down_sync(0xffffffffu, arg, o);
-        if (oa >= 0 && (arg < 0 || ob > best || (ob == best && oa < arg))) {
-          best = ob;
-          arg = oa;
-        }
-      }
-      if (lane == 0) {
-        s_best[warp] = best;
-        s_arg[warp] = arg;
-      }
-      __syncthreads();
-      if (t == 0) {
-        double bb = -1.0;
-        int ba = -1;
-        for (int q = 0; q < nt / 32; ++q) {
-          const int oa = s_arg[q];
-          const double ob = s_best[q];
-          if (oa >= 0 && (ba < 0 || ob > bb || (ob == bb && oa < ba))) {
-            bb = ob;
-            ba = oa;
-          }
-        }
-        // a NaN never compares larger, so an all-NaN or all-zero column fails here
-        s_arg[0] = (ba >= 0 && fabs(colk[ba]) > 0.0) ? ba : -1;
-      }
-      __syncthreads();
-      const int p = s_arg[0];
-      if (p >= 0) {
-        const double piv = colk[p];
-        for (int i = k + 1 + t; i < n; i += nt) {
-          const double v = (i == p) ? colk[k] : colk[i];
-          const double l = v / piv;
-          for (int r = 0; r < cs; ++r) dir_store_remote(dir_remote(lbuf + size_t(par) * n + i, r), l);
-        }
-      }
-      if (t < cs) dir_store_remote(dir_remote(s_piv + par, t), p);
-    }
-    dir_cluster_sync();
+    const int par = k & 1;
+    dir_cluster_wait();
     const int p = s_piv[par];
     if (p < 0) {
       if (me == 0 && t == 0) status[0] = 0;
       return;  // every CTA returns here, after the last remote store
     }
+    const bool below = t > k && t < n;
+    const double li = below ? lbuf[size_t(par) * n + t] : 0.0;
+    __syncthreads();  // the step before's updates
     if (p != k) {
       for (int s = t; s < cnt; s += nt) {
         double* c = A + size_t(s) * n;
@@ -195,35 +211,42 @@ __global__ void __launch_bounds__(kDirThreads) k_direct_lu(int n, const double* 
         s_perm[k] = s_perm[p];
         s_perm[p] = q;
       }
+      __syncthreads();
     }
-    __syncthreads();
-    const double* l = lbuf + size_t(par) * n;
-    if (me == owner) {
-      double* colk = A + size_t(k / cs) * n;
-      for (int i = k + 1 + t; i < n; i += nt) colk[i] = l[i];
+    if (me == k % cs && below) A[size_t(k / cs) * n + t] = li;
+    if (k + 1 == n) break;
+    // rank-1 update of the local columns j > k, the next pivot column first
+    int s0 = k >= me ? (k - me) / cs + 1 : 0;
+    if (me == (k + 1) % cs) {
+      double* c = A + size_t(s0) * n;
+      const double u = c[k];
+      double v = t < n ? c[t] : 0.0;
+      if (below && (DENSE || (u != 0.0 && li != 0.0))) {
+        v = v - li * u;
+        c[t] = v;
+      }
+      publish(k + 1, v);
+      ++s0;
     }
-    // rank-1 update of the local columns j > k
-    const int s0 = k >= me ? (k - me) / cs + 1 : 0;
-    const int m = n - k - 1;
-    if (m > 0 && s0 < cnt) {
-      const int total = (cnt - s0) * m;
-      for (int idx = t; idx < total; idx += nt) {
-        const int s = s0 + idx / m, i = k + 1 + idx % m;
+    dir_cluster_arrive();
+    if (below && (DENSE || li != 0.0)) {
+#pragma unroll 4
+      for (int s = s0; s < cnt; ++s) {
         double* c = A + size_t(s) * n;
         const double u = c[k];
-        if (u == 0.0) continue;
-        const double li = l[i];
-        if (li != 0.0) c[i] = c[i] - li * u;
+        if (DENSE || u != 0.0) c[t] = c[t] - li * u;
       }
     }
-    __syncthreads();
+    __syncwarp();
   }
-  for (int idx = t; idx < cnt * n; idx += nt) {
-    const int s = idx / n, i = idx % n, j = s * cs + me;
-    lu[size_t(j) * n + i] = A[idx];
-  }
+  __syncthreads();
+  for (int s = 0; s < cnt; ++s)
+    if (t < n) {
+      const int j = s * cs + me;
+      (DENSE ? lu[size_t(t) * n + j] : lu[size_t(j) * n + t]) = A[size_t(s) * n + t];
+    }
   if (me == 0) {
-    for (int i = t; i < n; i += nt) perm[i] = s_perm[i];
+    if (t < n) perm[t] = s_perm[t];
     if (t == 0) status[0] = 1;
   }
 }
@@ -328,6 +351,31 @@ __global__ void __launch_bounds__(kDirThreads) k_direct_residual(int n, const do
 
 }  // namespace
 
+// LU of a coarse pressure matrix (n <= kDenseCoarseCells rows, row-major, in place) on a cluster of at
+// most eight CTAs, each with at most 38 columns.
+void dense_lu_launch(int n, double* a, int* perm, int* ok, cudaStream_t stream) {
+  constexpr int most = (kDenseCoarseCells + 7) / 8 + 2;  // columns and two rows of multipliers
+  const void* fn = (const void*)k_direct_lu<true>;
+  // a constant, so that no caller lowers another's limit
+  cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(double)) * most * kDenseCoarseCells);
+  int cs = 1;
+  while (cs < 8 && (n + cs - 1) / cs > 32) cs *= 2;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(cs);
+  cfg.blockDim = dim3(kDirThreads);
+  cfg.dynamicSmemBytes = sizeof(double) * ((size_t(n) + cs - 1) / cs + 2) * n;
+  cfg.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = cs;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  void* args[] = {&n, &a, &a, &perm, &ok};
+  cudaLaunchKernelExC(&cfg, fn, args);
+}
+
 int direct_rows(const Ctx& c, bool with_wells) {
   return 3 * c.n + (with_wells ? c.topo.n_wells + c.topo.n_perfs : 0);
 }
@@ -348,34 +396,37 @@ static void ensure_direct_workspace(Ctx& c, int nf) {
   int optin = 0;
   RF_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c.device));
   cudaFuncAttributes fa;
-  RF_CUDA(cudaFuncGetAttributes(&fa, (const void*)k_direct_lu));
+  RF_CUDA(cudaFuncGetAttributes(&fa, (const void*)k_direct_lu<false>));
   c.dir_cs = 0;
-  for (int cs = 1; cs <= 16; cs *= 2) {
-    const int ncl = (nf + cs - 1) / cs;
-    const size_t bytes = sizeof(double) * (size_t(ncl) * nf + 2 * size_t(nf));
-    if (bytes + fa.sharedSizeBytes > size_t(optin)) continue;
-    if (bytes > 48 * 1024)
-      RF_CUDA(cudaFuncSetAttribute((const void*)k_direct_lu, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   int(bytes)));
-    if (cs > 8) RF_CUDA(cudaFuncSetAttribute((const void*)k_direct_lu, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(cs);
-    cfg.blockDim = dim3(kDirThreads);
-    cfg.dynamicSmemBytes = bytes;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = cs;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    int ncl_active = 0;
-    if (cudaOccupancyMaxActiveClusters(&ncl_active, (const void*)k_direct_lu, &cfg) == cudaSuccess && ncl_active >= 1) {
-      c.dir_cs = cs;
-      c.dir_smem = bytes;
-      break;
+  // the smallest cluster that leaves a CTA at most 32 columns (their update then ends within the
+  // barrier), else the smallest whose columns fit
+  for (int pass = 0; pass < 2 && c.dir_cs == 0; ++pass)
+    for (int cs = 1; cs <= 16; cs *= 2) {
+      const int ncl = (nf + cs - 1) / cs;
+      if (pass == 0 && ncl > 32) continue;
+      const size_t bytes = sizeof(double) * (size_t(ncl) * nf + 2 * size_t(nf));
+      if (bytes + fa.sharedSizeBytes > size_t(optin)) continue;
+      if (bytes > 48 * 1024)
+        raise_dynamic_smem((const void*)k_direct_lu<false>, bytes);
+      if (cs > 8) RF_CUDA(cudaFuncSetAttribute((const void*)k_direct_lu<false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(cs);
+      cfg.blockDim = dim3(kDirThreads);
+      cfg.dynamicSmemBytes = bytes;
+      cudaLaunchAttribute at[1];
+      at[0].id = cudaLaunchAttributeClusterDimension;
+      at[0].val.clusterDim.x = cs;
+      at[0].val.clusterDim.y = 1;
+      at[0].val.clusterDim.z = 1;
+      cfg.attrs = at;
+      cfg.numAttrs = 1;
+      int ncl_active = 0;
+      if (cudaOccupancyMaxActiveClusters(&ncl_active, (const void*)k_direct_lu<false>, &cfg) == cudaSuccess && ncl_active >= 1) {
+        c.dir_cs = cs;
+        c.dir_smem = bytes;
+        break;
+      }
     }
-  }
   cudaGetLastError();
   if (c.dir_cs == 0) throw CudaError("no thread-block cluster shape fits the direct LU of " + std::to_string(nf) + " rows");
 }
@@ -432,7 +483,7 @@ LinResult linear_solve_direct(Ctx& c, bool with_wells, std::vector<double>* h_dx
     int nn = nf;
     const double* ain = A;
     void* args[] = {&nn, &ain, &LU, &perm, &status};
-    RF_CUDA(cudaLaunchKernelExC(&cfg, (const void*)k_direct_lu, args));
+    RF_CUDA(cudaLaunchKernelExC(&cfg, (const void*)k_direct_lu<false>, args));
     c.launches++;
   }
   k_direct_solve<<<1, kDirThreads, 0, c.stream>>>(nf, LU, perm, b, x, status + 1);

@@ -1691,101 +1691,12 @@ __global__ void k_dense_build(int nb, const int* __restrict__ rp, const int* __r
 // |pivot| of the column wins, multipliers are scaled by the pivot's reciprocal, updates are
 // y = (-p) * c + y, the forward solve has a unit diagonal and the back substitution applies the
 // columns from the last one down.  Two kernels:
-//   k_dense_lu: one 1024-thread block factors `a` in place (row-major).  A warp owns a row of the
-//     trailing matrix at each step, its lanes the columns; while updating, lane 0 of each warp
-//     also tracks the largest |a_r,c+1| of its rows, so the next pivot is a reduction over 32
-//     partials (value descending, row ascending: the sequential scan's first maximum) instead of
-//     a pass over the column.  ok[0] = 0 when a pivot is exactly zero, else 1.
+//   the LU (rf_direct.cu, dense_lu_launch) factors `a` in place (row-major); ok[0] = 0 when a pivot is
+//     exactly zero, else 1.
 //   k_dense_inv_cols: thread block b solves for the 32 columns 32b.. of the inverse with them held
 //     in shared memory (lane = column, warp = row), the factors read from global memory.
 // `perm` holds n ints.
 constexpr int kDenseColsPerBlock = 32;
-
-__device__ __forceinline__ void piv_better(double v, int r, double& bv, int& br) {
-  if (br < 0 || v > bv || (v == bv && r < br)) {
-    bv = v;
-    br = r;
-  }
-}
-
-__global__ void __launch_bounds__(1024) k_dense_lu(int n, double* a, int* perm, int* ok) {
-  __shared__ double s_val[32];
-  __shared__ int s_row[32];
-  const int t = threadIdx.x, lane = t & 31, warp = t >> 5, nwarps = blockDim.x >> 5;
-  for (int r = t; r < n; r += blockDim.x) perm[r] = r;
-  // partial pivots of column 0
-  {
-    double bv = 0.0;
-    int br = -1;
-    for (int r = t; r < n; r += blockDim.x) piv_better(fabs(a[size_t(r) * n]), r, bv, br);
-    for (int o = 16; o > 0; o >>= 1) {
-      const double ov = __shfl_down_sync(0xffffffffu, bv, o);
-      const int orr = __shfl_down_sync(0xffffffffu, br, o);
-      if (orr >= 0) piv_better(ov, orr, bv, br);
-    }
-    if (lane == 0) {
-      s_val[warp] = bv;
-      s_row[warp] = br;
-    }
-  }
-  __syncthreads();
-  for (int c = 0; c < n; ++c) {
-    // every warp reduces the warps' partials (lane w takes warp w's) by the same butterfly and
-    // takes lane 0's result: the same pivot everywhere.  piv_better is a total order (largest
-    // value, then smallest row), so the order of the reduction does not change the pivot.
-    double bv = 0.0;
-    int piv = -1;
-    if (lane < nwarps && s_row[lane] >= 0) {
-      bv = s_val[lane];
-      piv = s_row[lane];
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const double ov = __shfl_xor_sync(0xffffffffu, bv, o);
-      const int orr = __shfl_xor_sync(0xffffffffu, piv, o);
-      if (orr >= 0) piv_better(ov, orr, bv, piv);
-    }
-    bv = __shfl_sync(0xffffffffu, bv, 0);
-    piv = __shfl_sync(0xffffffffu, piv, 0);
-    if (piv < 0 || bv == 0.0) {  // |a_piv,c| of the partials: an exactly zero pivot
-      if (t == 0) ok[0] = 0;
-      return;  // uniform: every thread saw the same partials
-    }
-    if (piv != c) {
-      for (int k = t; k < n; k += blockDim.x) {
-        const double x = a[size_t(c) * n + k];
-        a[size_t(c) * n + k] = a[size_t(piv) * n + k];
-        a[size_t(piv) * n + k] = x;
-      }
-      if (t == 0) {
-        const int q = perm[c];
-        perm[c] = perm[piv];
-        perm[piv] = q;
-      }
-    }
-    __syncthreads();  // swapped rows visible; every thread is done reading this step's partials
-    const double inv_pivot = 1.0 / a[size_t(c) * n + c];
-    double wv = 0.0;
-    int wr = -1;
-    for (int r = c + 1 + warp; r < n; r += nwarps) {
-      double* row = a + size_t(r) * n;
-      const double m = row[c] * inv_pivot;
-      __syncwarp();
-      if (lane == 0) row[c] = m;
-      for (int k = c + 1 + lane; k < n; k += 32) {
-        const double p = -a[size_t(c) * n + k];
-        row[k] = p * m + row[k];
-      }
-      if (lane == 0 && c + 1 < n) piv_better(fabs(row[c + 1]), r, wv, wr);
-    }
-    if (lane == 0) {
-      s_val[warp] = wv;
-      s_row[warp] = wr;
-    }
-    __syncthreads();
-  }
-  if (t == 0) ok[0] = 1;
-}
 
 __global__ void __launch_bounds__(1024) k_dense_inv_cols(int n, const double* __restrict__ lu,
                                                          const int* __restrict__ perm, const int* __restrict__ ok,
@@ -1820,7 +1731,7 @@ void dense_invert_launch(int n, double* a, double* inv, int* perm, int* ok, cuda
     cudaFuncSetAttribute((const void*)k_dense_inv_cols, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          int(sizeof(double) * 299 * kDenseColsPerBlock));
   });
-  k_dense_lu<<<1, 1024, 0, stream>>>(n, a, perm, ok);
+  dense_lu_launch(n, a, perm, ok, stream);
   k_dense_inv_cols<<<(n + kDenseColsPerBlock - 1) / kDenseColsPerBlock, 1024, smem, stream>>>(n, a, perm, ok, inv);
 }
 

@@ -6,7 +6,7 @@
 // cudaFree can synchronise the device.  For them this file offers x = A^{-1} b for a dense
 // row-major n x n pressure matrix, n <= RF_NOALLOC_MAX_ROWS (299, the size up to which the
 // reference's CPR inverts its pressure block densely, gmres_block_jacobi.rs:903-917).  It runs
-// the same kernels as a context's CPR coarse stage (k_dense_lu and k_dense_inv_cols, the inverse
+// the same kernels as a context's CPR coarse stage (dense_lu_launch and k_dense_inv_cols, the inverse
 // by LU with partial pivoting in nalgebra's order, then k_dense_matvec), with all scratch (the LU
 // work copy, the inverse, the row permutation and a status word) in one file-scope static device
 // array.  The caller passes A, b

@@ -64,6 +64,10 @@ int direct_rows(const Ctx& c, bool with_wells);
 // residual stays above 1e-12 + 5e-3 |b|.
 LinResult linear_solve_direct(Ctx& c, bool with_wells, std::vector<double>* h_dx_tail);
 
+// LU with partial pivoting of a coarse pressure matrix (rf_direct.cu); launch errors are left to
+// cudaGetLastError.
+void dense_lu_launch(int n, double* a, int* perm, int* ok, cudaStream_t stream);
+
 // Discrete adjoint tape hooks of the outer controller (rf_adjoint.cu); no-ops unless recording.
 void adjoint_on_step_begin(Ctx& c);
 void adjoint_on_substep_accepted(Ctx& c, double dt);
