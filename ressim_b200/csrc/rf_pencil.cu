@@ -25,7 +25,8 @@
 //     warp between two barriers, their products formed by one lane each.
 // What bounds it: the chain of steps.  Cycles per step (B200, FP64): 203 forward and 242 backward
 // with five line warps, 154 and 187 with one, 300-400 with the hand-over between CTAs, against some
-// 1,430 before.  Report steps before and after: 45x61x7 waterflood 175 -> 102 ms, 60x60x20 black oil
+// 1,430 before.  Report steps with the kernel it replaces and with its first form, the other kernels
+// as they were then: 45x61x7 waterflood 175 -> 102 ms, 60x60x20 black oil
 // 125 -> 66, 127x101x40 waterflood 1,617 -> 363 (mixed 1,581 -> 364), a 16-variant ensemble's 1,489
 // -> 878; one linear solve on 40x31x5 25.5 -> 12.8 ms.  Factors and vectors come from L2.
 // Every row takes the operations of the reference's sequential sweep in its order.  Dot products
@@ -286,7 +287,8 @@ __device__ __forceinline__ int tag_of(float v) { return __float_as_int(v); }
 // y_lo ~ 1/d - y is within half an ulp and a little.  The guards (and the pivot's range in
 // pen_recip) keep every intermediate normal.
 // FP32: s * RN64(1/d) in FP64 is within 2^-52 of s/d, and a quotient of two 24-bit numbers lies at
-// least 2^-49 (relative) from any rounding boundary of FP32, so its rounding is RN32(s/d).
+// least 2^-49 (relative) from any rounding boundary of FP32, so its rounding is RN32(s/d) (a quotient
+// below FP32's normal range may round a tie the other way: 2^-149 at most).
 __device__ __forceinline__ double pen_div(double s, double d, double rd, bool& ok) {
   const double rlo = __fma_rn(-d, rd, 1.0) * rd;
   const double q = __fma_rn(s, rd, s * rlo);
