@@ -1396,7 +1396,7 @@ void layout_for(Ctx& c, int cs) {
   zeros(P.d_rd, m);
   zeros(P.d_work, 10 * sizeof(double) * m);
   RF_CUDA(cudaDeviceSynchronize());
-  P.packed = -1;
+  P.packed = P.typed = -1;
 }
 
 // The slots of the dot products' elements, virtual warp by virtual warp, for the order the solve's
@@ -1558,6 +1558,16 @@ bool pencil_active(const Ctx& c) {
 
 void pencil_pack(Ctx& c) {
   PencilPlan& P = c.pen;
+  const int f = c.precision == 1 ? 1 : 0;
+  // The sweeps rely on zeros in the slots outside the lines, and the buffers hold either value type: what
+  // the other one left there would be read as factors and vectors (halves of doubles, some of them
+  // NaN).  The solves' vectors keep their zeros from one solve to the next.
+  if (P.typed >= 0 && P.typed != f) {
+    for (auto* b : {&P.d_lrec, &P.d_brec, &P.d_arec})
+      RF_CUDA(cudaMemsetAsync(b->p, 0, sizeof(double) * b->n, c.stream));
+    RF_CUDA(cudaMemsetAsync(P.d_work.p, 0, P.d_work.n, c.stream));
+  }
+  P.typed = f;
   auto go = [&](auto zero) {
     using T = decltype(zero);
     PenPack<T> a;
@@ -1590,7 +1600,7 @@ void pencil_pack(Ctx& c) {
   else
     go(0.0);
   c.launches++;
-  P.packed = c.precision == 1 ? 1 : 0;
+  P.packed = f;
 }
 
 static_assert(sizeof(PenArgs<double>) <= kBatchArgBytes, "batched launch arguments must fit a batch item");
