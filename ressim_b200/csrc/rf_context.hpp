@@ -117,7 +117,8 @@ struct PencilPlan {
   std::set<std::pair<int, int>> fill_cols;  // columns (j, j') joined by a well's fill
   std::vector<int> h_spec_row, h_spec_col_row, h_nat, dots_key;  // dots_key: the order d_list holds
   DBuf<int> d_cta, d_nat, d_rec_at, d_rec_half, d_list_ptr, d_list[3], d_spec_slot, d_spec_ptr, d_spec_col, d_spec_map;
-  DBuf<int> d_well_cta, d_well_at, d_well_slot, d_well_ptr, d_well_row, d_well_map;
+  DBuf<int> d_well_cta, d_well_slot, d_well_ptr, d_well_row, d_well_map;
+  DBuf<int2> d_well_at;
   DBuf<unsigned short> d_well_code;
   // values, sized for double and holding either type
   DBuf<double> d_well_val, d_well_piv, d_spec_val, d_lrec, d_brec, d_arec, d_rd;

@@ -84,10 +84,10 @@ struct PenArgs {
   const int* spec_ptr;
   const int* spec_col;  // slots
   const T* spec_val;
-  // the same rows in the sweeps: first one of each CTA, (step, line) packed, slot, entry ranges per
+  // the same rows in the sweeps: first one of each CTA, step and line, slot, entry ranges per
   // direction, entry codes (window index, or 0x8000 + listed row of the CTA) and values
   const int* well_cta;   // [cs + 1]
-  const int* well_at;    // [nspec] step << 16 | line
+  const int2* well_at;   // [nspec] {step, line}
   const int* well_slot;  // [nspec]
   const int* well_ptr;   // [2][nspec + 1]
   const unsigned short* well_code;
@@ -522,9 +522,8 @@ __device__ __noinline__ void pen_send(const PenSweep<T>& w, const T* in) {
   auto next_row = [&]() {
     at = -1;
     if (e < 0 || e >= nwell) return;
-    const int packed = lds_i(w.at + 4u * unsigned(e));
-    at = packed >> 16;
-    line = B * unsigned(packed & 0xffff);
+    at = lds_i(w.at + 8u * unsigned(e));
+    line = B * unsigned(lds_i(w.at + 8u * unsigned(e) + 4u));
     const unsigned ptr = w.ptr + 4u * unsigned(FWD ? e : nwell + 1 + e);
     e0 = lds_i(ptr);
     cnt = lds_i(ptr + 4) - e0;
@@ -841,7 +840,7 @@ __device__ void pen_body(const PenArgs<T>& a, unsigned char* raw) {
   for (int e = tid; e < 2 * a.chunk * P; e += nt) reinterpret_cast<T*>(raw + o.rows)[e] = T(0);
   for (int e = tid; e <= 2 * nz; e += nt) reinterpret_cast<T*>(raw + o.ghost)[e] = T(0);
   for (int e = tid; e < nwell; e += nt) {
-    reinterpret_cast<int*>(raw + o.at)[e] = a.well_at[w0 + e];
+    reinterpret_cast<int2*>(raw + o.at)[e] = a.well_at[w0 + e];
     reinterpret_cast<int*>(raw + o.slot)[e] = a.well_slot[w0 + e];
     reinterpret_cast<T*>(raw + o.piv)[e] = a.well_piv[w0 + e];
   }
@@ -1279,12 +1278,13 @@ void layout_for(Ctx& c, int cs) {
     return bx != by ? bx < by : step_of(x) < step_of(y);
   });
   const int ns = int(ord.size());
-  std::vector<int> well_cta(cs + 1, 0), at(ns), slot(ns), ptr(2 * (size_t(ns) + 1)), map, number(n, -1);
+  std::vector<int> well_cta(cs + 1, 0), slot(ns), ptr(2 * (size_t(ns) + 1)), map, number(n, -1);
+  std::vector<int2> at(ns);
   std::vector<unsigned short> code;
   for (int e = 0; e < ns; ++e) {
     const int b = owner[(ord[e] / nx) % ny];
     well_cta[b + 1]++;
-    at[e] = step_of(ord[e]) << 16 | line_of(ord[e]);
+    at[e] = make_int2(step_of(ord[e]), line_of(ord[e]));
     slot[e] = nat[ord[e]];
   }
   for (int b = 0; b < cs; ++b) well_cta[b + 1] += well_cta[b];
@@ -1490,9 +1490,10 @@ void pencil_replan(Ctx& c) {
 void free_pencil_plan(Ctx& c) {
   PencilPlan& P = c.pen;
   for (auto* b : {&P.d_cta, &P.d_nat, &P.d_rec_at, &P.d_rec_half, &P.d_spec_slot, &P.d_spec_ptr, &P.d_spec_col,
-                  &P.d_spec_map, &P.d_well_cta, &P.d_well_at, &P.d_well_slot, &P.d_well_ptr, &P.d_well_row,
-                  &P.d_well_map, &P.d_list_ptr, &P.d_list[0], &P.d_list[1], &P.d_list[2]})
+                  &P.d_spec_map, &P.d_well_cta, &P.d_well_slot, &P.d_well_ptr, &P.d_well_row, &P.d_well_map,
+                  &P.d_list_ptr, &P.d_list[0], &P.d_list[1], &P.d_list[2]})
     b->free();
+  P.d_well_at.free();
   P.d_well_code.free();
   for (auto* b : {&P.d_well_val, &P.d_well_piv, &P.d_spec_val, &P.d_lrec, &P.d_brec, &P.d_arec, &P.d_rd}) b->free();
   for (auto* b : {&P.d_special, &P.d_work}) b->free();

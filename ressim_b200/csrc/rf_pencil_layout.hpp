@@ -59,7 +59,7 @@ RF_PEN_HD inline PenLayout pen_layout(int nx, int nz, int cols, int cs, int chun
   o.well_y = take(size_t(wells) * sizeof(T));
   o.well_x = take(size_t(wells) * sizeof(T));
   o.piv = take(size_t(wells) * sizeof(T));
-  o.at = take((size_t(wells) + 1) * sizeof(int));
+  o.at = take(size_t(wells) * 2 * sizeof(int));
   o.slot = take(size_t(wells) * sizeof(int));
   o.ptr = take(2 * (size_t(wells) + 1) * sizeof(int));
   o.val = take(size_t(entries) * sizeof(T));
