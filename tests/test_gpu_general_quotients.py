@@ -3,7 +3,8 @@
 Such a sweep of the pressure solve along grid lines is repeated with IEEE divisions, and the solve goes
 on with them, on every CTA of the cluster.  The systems below reach that with finite results: values
 that decay below 1e-250 away from the one source, on one CTA and on several, without wells and with
-wells in some of the CTAs only.  Results equal the level-order kernel's bit for bit: no tolerance.
+wells in some of the CTAs only, and a pivot beyond 1e30 whose row the first attempt leaves as a NaN
+in the repeated sweep's first rows.  Results equal the level-order kernel's bit for bit: no tolerance.
 """
 import numpy as np
 import pytest
@@ -59,3 +60,18 @@ def test_values_that_decay_below_the_range(dims, wells, end, precision):
     rhs = np.zeros(3 * int(np.prod(dims)))
     rhs.reshape(-1, 3)[end] = 1.0
     _solve_both(dims, ptr, col, val, rhs, precision, wells)
+
+
+@pytest.mark.parametrize("dims,cell", [((13, 12, 5), 400), ((13, 12, 5), 403), ((40, 31, 4), 2100), ((350, 1, 1), 200)])
+def test_a_pivot_above_the_range(dims, cell):
+    """Couplings of 1e18 in both directions between two neighbours along x make the second one's pivot
+    about -1e35."""
+    rng = np.random.default_rng(5)
+    ptr, row, col = _pattern(*dims)
+    val = rng.uniform(-0.1, 0.1, (len(col), 3, 3))
+    on = row == col
+    val[on] += np.eye(3) * rng.uniform(6.0, 9.0, (int(on.sum()), 1, 1))
+    val[~on, 0, 0] = -rng.uniform(0.1, 0.9, int((~on).sum()))
+    val[(row == cell) & (col == cell + 1), 0, 0] = 1e18
+    val[(row == cell + 1) & (col == cell), 0, 0] = 1e18
+    _solve_both(dims, ptr, col, val, rng.standard_normal(3 * int(np.prod(dims))))
