@@ -627,6 +627,14 @@ __device__ __forceinline__ void pen_sweep(const PenSweep<T>& w, unsigned phase0,
   }
 }
 
+// Zeros in the result rows and the neighbour's columns, which lines outside their cells read times zero.
+template <class T>
+__device__ __noinline__ void pen_clear(const PenSweep<T>& w) {
+  constexpr unsigned B = sizeof(T);
+  for (int e = threadIdx.x; e < 2 * w.chunk * w.stride; e += kPenThreads) sts(w.rows + B * unsigned(e), T(0));
+  for (int e = threadIdx.x; e < 2 * w.nz; e += kPenThreads) sts(w.ghost + B * unsigned(e), T(0));
+}
+
 // out = A in on the CTA's cells.  A thread takes part of a line: the x neighbours come from its own
 // loads, the y and z ones at constant distances (in a neighbouring CTA's region with its own).  Rows
 // with entries outside the stencil take a warp each.
@@ -837,13 +845,8 @@ __device__ void pen_body(const PenArgs<T>& a, unsigned char* raw) {
   const PenLayout o = pen_layout<T>(nx, nz, cols, g.cs, a.chunk, nvw, nwell, f1 - f0 + b1 - b0);
   double* const red_base = reinterpret_cast<double*>(raw + o.red);
   const unsigned bad_at = pen_smem(raw + o.bad);
-  // Result rows and the neighbour's columns, which lines outside their cells read times zero: finite
-  // from the start and after any sweep that the solve goes on from.
-  auto clear_rows = [&]() {
-    for (int e = tid; e < 2 * a.chunk * P; e += nt) reinterpret_cast<T*>(raw + o.rows)[e] = T(0);
-    for (int e = tid; e <= 2 * nz; e += nt) reinterpret_cast<T*>(raw + o.ghost)[e] = T(0);
-  };
-  clear_rows();
+  for (int e = tid; e < 2 * a.chunk * P; e += nt) reinterpret_cast<T*>(raw + o.rows)[e] = T(0);
+  for (int e = tid; e <= 2 * nz; e += nt) reinterpret_cast<T*>(raw + o.ghost)[e] = T(0);
   for (int e = tid; e < nwell; e += nt) {
     reinterpret_cast<int2*>(raw + o.at)[e] = a.well_at[w0 + e];
     reinterpret_cast<int*>(raw + o.slot)[e] = a.well_slot[w0 + e];
@@ -989,7 +992,7 @@ __device__ void pen_body(const PenArgs<T>& a, unsigned char* raw) {
         pen_sync(g.cs);
         if (general || lds_i(bad_at) == 0) break;
         general = true;
-        clear_rows();  // the attempt may have left NaNs: pen_div of a pivot that pen_recip refuses
+        pen_clear(sweep[1]);  // the attempt may have left NaNs: pen_div of a pivot that pen_recip refuses
         __syncthreads();
       }
       pen_spmv<T>(a, gs, mp, ap);
