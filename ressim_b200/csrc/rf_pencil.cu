@@ -42,6 +42,7 @@
 #include "rf_fiber.hpp"
 #include "rf_ops.hpp"
 #include "rf_pencil_layout.hpp"
+#include "rf_quotient.hpp"
 
 namespace rf {
 
@@ -227,34 +228,6 @@ __device__ __forceinline__ void ld4(const float* p, float& a, float& b, float& c
 }
 __device__ __forceinline__ int tag_of(double v) { return __double2loint(v); }
 __device__ __forceinline__ int tag_of(float v) { return __float_as_int(v); }
-
-// s / d from rd, the correctly rounded reciprocal of d; `ok` false: the quotient needs the general
-// division.
-// FP64: Markstein's theorem (IBM J. Res. Dev. 34, 1990): with y = RN(1/d) and q within one ulp of
-// s/d, r = s - d q is exact and RN(q + r y) = RN(s/d).  q = RN(s y + RN(s y_lo)) with
-// y_lo ~ 1/d - y is within half an ulp and a little.  The guards (and the pivot's range in
-// pen_recip) keep every intermediate normal.
-// FP32: s * RN64(1/d) in FP64 is within 2^-52 of s/d, and a quotient of two 24-bit numbers lies at
-// least 2^-49 (relative) from any rounding boundary of FP32, so its rounding is RN32(s/d) (a quotient
-// below FP32's normal range may round a tie the other way: 2^-149 at most).
-__device__ __forceinline__ double pen_div(double s, double d, double rd, bool& ok) {
-  const double rlo = __fma_rn(-d, rd, 1.0) * rd;
-  const double q = __fma_rn(s, rd, s * rlo);
-  const double r = __fma_rn(-d, q, s);
-  const double m = fabs(s);
-  ok = m < 1e250 && (m > 1e-250 || m == 0.0) && rd == rd;
-  return __fma_rn(r, rd, q);
-}
-__device__ __forceinline__ float pen_div(float s, float, double rd, bool& ok) {
-  ok = rd == rd;
-  return float(double(s) * rd);
-}
-// Pivots whose reciprocal or residual could leave the normal range take the general division.
-__device__ __forceinline__ double pen_recip(double d) {
-  const double m = fabs(d);
-  return m > 1e-30 && m < 1e30 ? 1.0 / d : __hiloint2double(0x7ff80000, 0);
-}
-__device__ __forceinline__ double pen_recip(float d) { return 1.0 / double(d); }
 
 // One direction's sweeps of one CTA; kept in shared memory.
 template <class T>
