@@ -109,6 +109,7 @@ struct PencilPlan {
   int cs = 0;           // CTAs the layout is for (0: none)
   int slots = 0, n_spec_entries = 0, n_well_entries = 0;
   int packed = -1;      // value type of the last packing (-1: none since the last factorisation)
+  int lost_message = -1;  // PenArgs::lost
   int typed = -1;       // value type the buffers hold (-1: zeros, which serve either)
   struct Listed {
     int j, entries;

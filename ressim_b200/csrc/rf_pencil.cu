@@ -20,7 +20,8 @@
 //   - the columns j are split over the cluster's CTAs.  One warp of each CTA sends the values of its
 //     last column (backward: first) to the next CTA with st.async, whose completion counts on an
 //     mbarrier per step there, another one receives them ahead of the line warps' barrier.
-//     Waits are bounded and set a status the host turns into an error;
+//     Waits are bounded (kPenWaitCycles); one that gives up sets a status the host turns into an error,
+//     and the cluster ends the solve after the sweep it is in;
 //   - rows with a well's fill (more entries, reaching far up the column) are solved by the sending
 //     warp between two barriers, their products formed by one lane each.
 // What bounds it: the chain of steps.  Cycles per step (B200, FP64): 203 forward and 242 backward
@@ -37,6 +38,7 @@
 // within one CTA's columns and the padding of the step order stays small; other decks, and callers
 // that name a kernel family, keep the level-list kernels.
 #include <algorithm>
+#include <cstdlib>
 #include <cstring>
 
 #include "rf_fiber.hpp"
@@ -54,6 +56,7 @@ constexpr int kPenLineWarps = 13;  // warps 0..12 own lines
 constexpr int kPenLoadWarp = 13;   // copies rows in and results out
 constexpr int kPenRecvWarp = 14, kPenSendWarp = 15;  // neighbours' values in; out, and the wells' rows
 constexpr int kPenLineThreads = 32 * kPenLineWarps;
+constexpr long long kPenWaitCycles = 2000000000;  // a second; a whole sweep takes some milliseconds
 constexpr unsigned kPenSpecial = 0x7ff80001u;            // high word of the reciprocal of a listed row
 
 // Order of a dot product: virtual threads (vblocks blocks of vwpb warps) each sum the elements
@@ -104,7 +107,9 @@ struct PenArgs {
   unsigned char* work; // slots doubles (iterate), then 9 vectors of `slots` T
   long long* iter_counter;
   int* status;
+  long long wait_limit;  // cycles
   int max_iters;
+  int lost;              // >= 0: the forward sweeps' message that never arrives complete (tests), else -1
 };
 
 // ---- small device helpers ----
@@ -202,17 +207,24 @@ __device__ __forceinline__ void st_async(unsigned addr, float v, unsigned mbar) 
                "r"(__float_as_int(v)), "r"(mbar)
                : "memory");
 }
-// bounded wait for the phase of parity `parity`; false when it gave up
-__device__ __forceinline__ bool mbar_wait_cluster(unsigned bar, unsigned parity) {
-  unsigned done = 0;
-  for (int it = 0; it < (1 << 20) && !done; ++it)
-    asm volatile(
-        "{\n\t.reg .pred q;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 q, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, q;\n\t}"
-        : "=r"(done)
-        : "r"(bar), "r"(parity)
-        : "memory");
+__device__ __forceinline__ bool mbar_try(unsigned bar, unsigned parity) {
+  unsigned done;
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 q, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(done)
+      : "r"(bar), "r"(parity)
+      : "memory");
   return done != 0;
+}
+// bounded wait for the phase of parity `parity`, a lane's own; false when it gave up
+__device__ __forceinline__ bool mbar_wait_cluster(unsigned bar, unsigned parity, const long long& limit) {
+  if (mbar_try(bar, parity)) return true;
+  const long long t0 = clock64(), most = limit;
+  do {
+    if (mbar_try(bar, parity)) return true;
+  } while (clock64() - t0 < most);
+  return false;
 }
 // four values of a constant array with one 32-byte (FP64) or 16-byte load; a 32-byte sector holds two
 // of the FP32 ones, so those stay in L1 for the second (without: 127x101x40, 77 -> 71 ms per solve)
@@ -236,11 +248,14 @@ struct PenSweep {
   const double* rd;    // reciprocals (backward)
   int* status;
   long long first;     // its slot
+  long long limit;     // cycles a wait may take
+  int lost;            // as in PenArgs
   int nx, nz, jc, steps, rounded, chunk, stride, ct, nbar, c, cs;
   int nwell;           // listed rows
   unsigned rows, ghost;                                                 // result rows, the neighbour's column
   unsigned place, full;                                                 // copied rows, their mbarriers
-  unsigned nbr, mbar, bad;                                              // neighbour's values and mbarriers
+  unsigned nbr, mbar;                                                   // neighbour's values and mbarriers
+  unsigned bad, gave;  // flags: a quotient needs the division; a wait gave up
   unsigned well_in, well_y, well_x, piv, at, slot, ptr, code, val;
 };
 // What the passes by slot and the reductions need of the CTA.
@@ -345,9 +360,19 @@ __device__ __noinline__ void pen_line(const PenSweep<T>& w) {
   if (!FWD && !GENERAL && bad) sts(w.bad, 1);
 }
 
+// All lanes of a warp of which a wait gave up.
+template <class T>
+__device__ __forceinline__ void pen_gave_up(const PenSweep<T>& w) {
+  if ((threadIdx.x & 31) != 0) return;
+  sts(w.gave, 1);
+  if (w.status) atomicExch(w.status, 3);
+}
+
 // The copying warp.  At the start of a chunk it writes the chunk before's results to `out` and
 // starts the copies of the next one in their places; before a chunk's last step it waits for the
 // next chunk (whose first row the line warps read then), and for the results' places to be free.
+// Once a wait has given up, here or in a sweep before, it starts no copies and waits for none, so that
+// no mbarrier is armed again before its phase has ended, and it ends after those in flight.
 template <class T, bool FWD>
 __device__ __noinline__ void pen_load(const PenSweep<T>& w, unsigned phase0, const T* in_, T* out_) {
   constexpr unsigned B = sizeof(T);
@@ -357,10 +382,14 @@ __device__ __noinline__ void pen_load(const PenSweep<T>& w, unsigned phase0, con
   const unsigned recs = w.place, ins = recs + unsigned(2 * G) * 4u * RB, rds = ins + unsigned(2 * G) * RB;
   const unsigned cb = unsigned(G) * RB, db = 8u * unsigned(G) * unsigned(stride);
   // chunk number c of the sweep covers the rows [G k, G k + G), k = c or, backward, from the end
+  bool ok = lds_i(w.gave) == 0;  // the same for all lanes
+  unsigned open = 0;             // the halves whose copies have not been waited for
   auto issue = [&](int c) {
-    if (lane != 0 || c >= chunks) return;
+    if (!ok || c >= chunks) return;
     const int k = FWD ? c : chunks - 1 - c;
     const unsigned h = unsigned(k & 1), bar = full + 8u * h;
+    open |= 1u << h;
+    if (lane != 0) return;
     const long long row = (long long)k * G * stride;
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(5u * cb + (FWD ? 0u : db))
                  : "memory");
@@ -374,12 +403,14 @@ __device__ __noinline__ void pen_load(const PenSweep<T>& w, unsigned phase0, con
   };
   // phases of the two mbarriers: phase0 holds their parities at the start of the sweep
   unsigned par = phase0;
-  bool ok = true;
   auto wait = [&](int c) {
+    if (!ok) return;
     const unsigned h = unsigned((FWD ? c : chunks - 1 - c) & 1);
-    if (ok) ok = mbar_wait_cluster(full + 8u * h, (par >> h) & 1u);
+    const bool got = mbar_wait_cluster(full + 8u * h, (par >> h) & 1u, w.limit);
+    ok = __all_sync(0xffffffffu, got);
+    if (!ok) return;
     par ^= 1u << h;
-    __syncwarp();
+    open &= ~(1u << h);
   };
   issue(0);
   issue(1);
@@ -393,9 +424,11 @@ __device__ __noinline__ void pen_load(const PenSweep<T>& w, unsigned phase0, con
       // chunk c's results take the place of chunk c - 2's
       if (t == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
       pen_bar(nbar);
-      if (t == 0 && c > 0 && lane == 0) {
-        proxy_fence_shared();
-        write(c - 1);
+      if (t == 0 && c > 0) {
+        if (lane == 0) {
+          proxy_fence_shared();
+          write(c - 1);
+        }
         issue(c + 1);
       }
     }
@@ -406,11 +439,16 @@ __device__ __noinline__ void pen_load(const PenSweep<T>& w, unsigned phase0, con
     write(chunks - 1);
     asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   }
-  if (!__all_sync(0xffffffffu, ok) && lane == 0 && w.status) atomicExch(w.status, 3);
+  if (ok) return;
+  pen_gave_up(w);
+  for (unsigned h = 0; h < 2; ++h)
+    if ((open >> h) & 1u) mbar_wait_cluster(full + 8u * h, (par >> h) & 1u, w.limit);
+  __syncwarp();
 }
 
 // The receiving warp: before each step's barrier it waits for the neighbouring CTA's values of the
-// step before and puts them into the result row.  Lane k takes layer k (and k + 32, ...).
+// step before and puts them into the result row.  Lane k takes layer k (and k + 32, ...).  A lane whose
+// wait gave up waits no more in this sweep; all lanes take the same steps and barriers all the same.
 template <class T, bool FWD>
 __device__ __noinline__ void pen_recv(const PenSweep<T>& w, unsigned phase) {
   constexpr unsigned B = sizeof(T);
@@ -418,11 +456,11 @@ __device__ __noinline__ void pen_recv(const PenSweep<T>& w, unsigned phase) {
   for (int u = lane; u < NM; u += 32) {
     const int cnt = min(nz - 1, u) - max(0, u - nx + 1) + 1;  // lines k with 0 <= u - k < nx
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(w.mbar + 8u * unsigned(u)),
-                 "r"(unsigned(cnt * sizeof(T)))
+                 "r"(unsigned((FWD && u == w.lost ? cnt + 1 : cnt) * sizeof(T)))
                  : "memory");
   }
   __syncwarp();
-  bool ok = true;
+  bool ok = true;  // a lane's own
   // step b reads the values sent as number u: b, or backward b less the rounding to whole chunks
   const int skip = FWD ? 0 : rounded - w.steps;
   const int kk = FWD ? lane : nz - 1 - lane;  // place in the message
@@ -435,8 +473,8 @@ __device__ __noinline__ void pen_recv(const PenSweep<T>& w, unsigned phase) {
   const int steps = rounded - skip;
 #pragma unroll 1
   for (int u = 0; u < steps; ++u) {
-    if (u < NM && ok) {
-      ok = mbar_wait_cluster(mb, phase);
+    if (u < NM) {
+      if (ok) ok = mbar_wait_cluster(mb, phase, w.limit);
       if (lane < nz && unsigned(u - kk) < unsigned(nx)) sts(to, lds(from, T(0)));
       for (int k = lane + 32; k < nz; k += 32) {
         const int q = FWD ? k : nz - 1 - k;
@@ -451,7 +489,7 @@ __device__ __noinline__ void pen_recv(const PenSweep<T>& w, unsigned phase) {
     pen_bar(nbar);
   }
   pen_bar(nbar);
-  if (!__all_sync(0xffffffffu, ok) && lane == 0 && w.status) atomicExch(w.status, 3);
+  if (!__all_sync(0xffffffffu, ok)) pen_gave_up(w);
 }
 
 // The sending warp (of a CTA with listed rows, or a neighbour to send to): after each step's
@@ -796,8 +834,22 @@ __device__ __noinline__ double2 pen_dots(const DotOrder& o, const PenCta& g, dou
   return pen_totals(o, red, nvw, cs);
 }
 
+// After a wait gave up, when no CTA sends any more: waits, bounded, for the values still on their way
+// into this CTA.  phase_f, phase_b: parities of the last forward and backward sweep's mbarriers.
+template <class T>
+__device__ __noinline__ void pen_drain(const PenSweep<T>* w, unsigned phase_f, unsigned phase_b) {
+  const int NM = w[0].nx + w[0].nz - 1;
+  for (int m = threadIdx.x; m < NM; m += kPenThreads) {
+    if (w[0].c > 0) mbar_wait_cluster(w[0].mbar + 8u * unsigned(m), phase_f, w[0].limit);
+    if (w[0].c + 1 < w[0].cs) mbar_wait_cluster(w[1].mbar + 8u * unsigned(m), phase_b, w[0].limit);
+  }
+  __syncwarp();
+}
+
 template <class T>
 __device__ void pen_body(const PenArgs<T>& a, unsigned char* raw) {
+  // a solve that gave up has left its mark, which the host reads after the linear solve
+  if (a.status && *(const volatile int*)a.status != 0) return;
   __shared__ PenSweep<T> sweep[2];
   __shared__ PenCta shared_cta;
   PenCta g;
@@ -817,7 +869,7 @@ __device__ void pen_body(const PenArgs<T>& a, unsigned char* raw) {
   const int b0 = a.well_ptr[wells + 1 + w0], b1 = a.well_ptr[wells + 1 + w0 + nwell];
   const PenLayout o = pen_layout<T>(nx, nz, cols, g.cs, a.chunk, nvw, nwell, f1 - f0 + b1 - b0);
   double* const red_base = reinterpret_cast<double*>(raw + o.red);
-  const unsigned bad_at = pen_smem(raw + o.bad);
+  const unsigned bad_at = pen_smem(raw + o.bad), gave_at = bad_at + 4u;
   for (int e = tid; e < 2 * a.chunk * P; e += nt) reinterpret_cast<T*>(raw + o.rows)[e] = T(0);
   for (int e = tid; e <= 2 * nz; e += nt) reinterpret_cast<T*>(raw + o.ghost)[e] = T(0);
   for (int e = tid; e < nwell; e += nt) {
@@ -841,6 +893,7 @@ __device__ void pen_body(const PenArgs<T>& a, unsigned char* raw) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(pen_smem(raw + o.full) + 8u * unsigned(tid)) : "memory");
   if (tid == 0) {
     sts(bad_at, 0);
+    sts(gave_at, 0);
     shared_cta = g;
   }
   if (tid < 2) {
@@ -859,7 +912,8 @@ __device__ void pen_body(const PenArgs<T>& a, unsigned char* raw) {
     w.nbar = w.ct + 32 + ((tid == 0 ? below : above) ? 32 : 0) + (nwell > 0 || (tid == 0 ? above : below) ? 32 : 0);
     w.rows = pen_smem(raw + o.rows), w.ghost = pen_smem(raw + o.ghost);
     w.place = pen_smem(raw + o.place), w.full = pen_smem(raw + o.full);
-    w.nbr = pen_smem(raw + o.nbr), w.bad = bad_at;
+    w.nbr = pen_smem(raw + o.nbr), w.bad = bad_at, w.gave = gave_at;
+    w.limit = a.wait_limit, w.lost = a.lost;
     w.mbar = pen_smem(raw + o.mbar) + (tid == 0 ? 0u : 8u * unsigned(nx + nz - 1));
     w.well_in = pen_smem(raw + o.well_in), w.well_y = pen_smem(raw + o.well_y), w.well_x = pen_smem(raw + o.well_x);
     w.piv = pen_smem(raw + o.piv), w.at = pen_smem(raw + o.at), w.slot = pen_smem(raw + o.slot);
@@ -958,16 +1012,25 @@ __device__ void pen_body(const PenArgs<T>& a, unsigned char* raw) {
         ph_b ^= 1u;
         ph_c ^= flip;
         __syncthreads();
-        // any CTA's flag reaches all of them; then the sweep is repeated, and the solve goes on, in
-        // the general form
-        if (!general && lds_i(bad_at) != 0 && tid < g.cs)
-          asm volatile("st.shared::cluster.s32 [%0], 1;" ::"r"(pen_map(bad_at, unsigned(tid))) : "memory");
+        // any CTA's flags reach all of them.  `bad`: the sweep is repeated, and the solve goes on, in
+        // the general form; `gave`: the solve ends
+        if (tid < g.cs) {
+          if (!general && lds_i(bad_at) != 0)
+            asm volatile("st.shared::cluster.s32 [%0], 1;" ::"r"(pen_map(bad_at, unsigned(tid))) : "memory");
+          if (lds_i(gave_at) != 0)
+            asm volatile("st.shared::cluster.s32 [%0], 1;" ::"r"(pen_map(gave_at, unsigned(tid))) : "memory");
+        }
         pen_sync(g.cs);
+        if (lds_i(gave_at) != 0) {
+          stop = true;
+          break;
+        }
         if (general || lds_i(bad_at) == 0) break;
         general = true;
         pen_clear(sweep[1]);  // the attempt may have left NaNs: pen_div of a pivot that pen_recip refuses
         __syncthreads();
       }
+      if (stop) break;
       pen_spmv<T>(a, gs, mp, ap);
       pen_sync(g.cs);
       if (half == 0) {
@@ -1009,6 +1072,7 @@ __device__ void pen_body(const PenArgs<T>& a, unsigned char* raw) {
     rho_prev = rho;
     rho = d.y;
   }
+  if (lds_i(gave_at) != 0) pen_drain(sweep, ph_f ^ 1u, ph_b ^ 1u);
   pen_sync(g.cs);
   for (int i = na + tid; i < nb; i += nt) a.x[i] = xq[a.nat[i]];
   if (g.c == 0 && tid == 0 && a.iter_counter)
@@ -1404,6 +1468,10 @@ void build_pencil_plan(Ctx& c) {
   PencilPlan& P = c.pen;
   P.built = 0;
   P.cs = 0;
+  // RESSIM_LOST_MESSAGE=m (read when a context is set up) makes every receiving CTA wait, in the forward
+  // sweeps, for more than its m-th message holds, and shortens the limit: the tests' wait that runs out
+  const char* lost = std::getenv("RESSIM_LOST_MESSAGE");
+  P.lost_message = lost ? std::atoi(lost) : -1;
   const int n = c.n, nx = c.nx, ny = c.ny, nz = c.nz, L = c.levels.n_levels;
   // smaller decks take the dense inverse of the pressure matrix
   if (n <= kDenseCoarseCells || n >= (1 << 26) || L != nx + ny + nz - 2) return;
@@ -1598,6 +1666,8 @@ void launch_bicgstab_pencil(Ctx& c, const double* rhs, double* x) {
     a.work = P.d_work.p;
     a.iter_counter = c.d_bicg_iters;
     a.status = c.d_pipe_status.p;
+    a.lost = P.lost_message;
+    a.wait_limit = P.lost_message >= 0 ? kPenWaitCycles / 50 : kPenWaitCycles;
     a.max_iters = 50;
     const size_t smem = pen_smem_bytes<T>(c, cs, a.chunk, a.dot.vblocks * a.dot.vwpb);
     if (c.batched && fiber_file(kBatchPressure, f + 2 * (1 + log2_of(cs)), &a, sizeof(a), kPenThreads, smem)) return;
