@@ -115,8 +115,8 @@ struct PencilDots {
   int threads;  // per block
   int blocks, slice;
 };
-void build_pencil_plan(Ctx& c);
-void pencil_replan(Ctx& c);
+void build_pencil_plan(Ctx& c) noexcept;
+void pencil_replan(Ctx& c) noexcept;
 void free_pencil_plan(Ctx& c);
 bool pencil_active(const Ctx& c);
 void pencil_pack(Ctx& c);

@@ -1462,25 +1462,18 @@ void dot_lists(Ctx& c, const PencilDots& d) {
   P.dots_key = key;
 }
 
-}  // namespace
-
-void build_pencil_plan(Ctx& c) {
+// The rows outside the 7-point shape; false: the deck keeps the level-list kernels.
+bool pencil_structure(Ctx& c) {
   PencilPlan& P = c.pen;
-  P.built = 0;
-  P.cs = 0;
-  // RESSIM_LOST_MESSAGE=m (read when a context is set up) makes every receiving CTA wait, in the forward
-  // sweeps, for more than its m-th message holds, and shortens the limit: the tests' wait that runs out
-  const char* lost = std::getenv("RESSIM_LOST_MESSAGE");
-  P.lost_message = lost ? std::atoi(lost) : -1;
   const int n = c.n, nx = c.nx, ny = c.ny, nz = c.nz, L = c.levels.n_levels;
   // smaller decks take the dense inverse of the pressure matrix
-  if (n <= kDenseCoarseCells || n >= (1 << 26) || L != nx + ny + nz - 2) return;
+  if (n <= kDenseCoarseCells || n >= (1 << 26) || L != nx + ny + nz - 2) return false;
   const std::vector<int>& lp = c.levels.h_ptr;
   const std::vector<int>& rows = c.levels.h_rows;
   for (int l = 0; l < L; ++l)
     for (int q = lp[l]; q < lp[l + 1]; ++q) {
       const int r = rows[q];
-      if (r % nx + (r / nx) % ny + r / (nx * ny) != l) return;
+      if (r % nx + (r / nx) % ny + r / (nx * ny) != l) return false;
     }
   // rows with entries outside the stencil, or read by one (the pattern is symmetric)
   std::vector<unsigned char> special(n, 0);
@@ -1509,7 +1502,7 @@ void build_pencil_plan(Ctx& c) {
     }
     spec_ptr.push_back(int(spec_map.size()));
   }
-  if (P.h_spec_row.size() >= 0x7fff) return;
+  if (P.h_spec_row.size() >= 0x7fff) return false;
   P.n_spec_entries = int(spec_map.size());
   upload_to(P.d_special, special);
   upload_to(P.d_spec_ptr, spec_ptr);
@@ -1519,20 +1512,40 @@ void build_pencil_plan(Ctx& c) {
   for (int k = 0; k < 5; ++k) {
     P.fits[0][k] = P.fits[1][k] = -1;
   }
-  P.built = 1;
+  return true;
+}
+
+}  // namespace
+
+// Host or device memory that cannot be had, or any CUDA error, leaves the deck without the plan: the
+// solves keep the level-list kernels, and what failed for good shows in the calls after it.
+void build_pencil_plan(Ctx& c) noexcept {
+  PencilPlan& P = c.pen;
+  P.built = 0;
+  P.cs = 0;
+  // RESSIM_LOST_MESSAGE=m (read when a context is set up) makes every receiving CTA wait, in the forward
+  // sweeps, for more than its m-th message holds, and shortens the limit: the tests' wait that runs out
+  const char* lost = std::getenv("RESSIM_LOST_MESSAGE");
+  P.lost_message = lost ? std::atoi(lost) : -1;
+  try {
+    P.built = pencil_structure(c) ? 1 : 0;
+  } catch (const std::exception&) {
+    cudaGetLastError();
+    free_pencil_plan(c);
+  }
   pencil_replan(c);
 }
 
 // The layout for the CTAs the context's solves run on now (its precision, or joining an ensemble,
-// changes them).  Where its memory cannot be had, the solves keep the level-list kernels.
-void pencil_replan(Ctx& c) {
+// changes them).  Called from a destructor too.
+void pencil_replan(Ctx& c) noexcept {
   if (!c.pen.built) return;
-  const int cs = pencil_want(c);
   try {
+    const int cs = pencil_want(c);
     if (cs > 0 && cs != c.pen.cs) layout_for(c, cs);
     c.pen.cs = cs;
     if (cs > 0) dot_lists(c, pressure_dots(c));
-  } catch (const CudaError&) {
+  } catch (const std::exception&) {
     cudaGetLastError();
     free_pencil_plan(c);
   }
