@@ -263,8 +263,9 @@ int64_t rf_kernel_launches(const RfCtx* ctx);
  * out (may be NULL) receives up to n values, read before the enable/reset below take effect:
  * ms for assembly, well elimination, CPR build, pressure stage, block-ILU0 smoother, Krylov,
  * update, the BiCGStab kernel alone, the direct LU route; then the BiCGStab iteration total, the number of BiCGStab
- * launches timed, the block count of the reduced matrix, and 1 when the level-order kernels serve
- * the pressure stage (0: the cluster kernels).
+ * launches timed, the block count of the reduced matrix, the kernels that serve the pressure stage
+ * (2 along grid lines, 1 in level order, 0 the cluster kernels), the CTAs of a pressure solve, and those of
+ * a factorisation (its cluster in batched launches for a variant stepped in RF_BATCH_GROUPS mode).
  * enable > 0 switches the profiler on, 0 off, < 0 leaves it as is; reset != 0 zeroes the totals. */
 int32_t rf_profile(RfCtx* ctx, int32_t enable, int32_t reset, double* out, int32_t n);
 

@@ -75,5 +75,6 @@ EXPORTED_SYMBOLS = (
     "rf_set_linear_refinement",
 )
 
+PRESSURE_KERNELS = ("cluster", "level", "lines")  # rf_profile's code of the kernels serving the pressure stage
 PHASES = ("assembly", "well_elimination", "cpr_build", "pressure_stage", "block_ilu_smoother", "krylov", "update",
           "bicgstab_kernel", "direct_lu")

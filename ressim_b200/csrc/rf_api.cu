@@ -1625,7 +1625,10 @@ int32_t rf_profile(RfCtx* ctx, int32_t enable, int32_t reset, double* out, int32
       if (n > rf::kPhCount) out[rf::kPhCount] = double(it);
       if (n > rf::kPhCount + 1) out[rf::kPhCount + 1] = double(c.phase_count[rf::kPhBicgKernel]);
       if (n > rf::kPhCount + 2) out[rf::kPhCount + 2] = double(c.nnzb);
-      if (n > rf::kPhCount + 3) out[rf::kPhCount + 3] = rf::level_solver_active(c) ? 1.0 : 0.0;
+      const bool lines = rf::pencil_active(c), level = !lines && rf::level_solver_active(c);
+      if (n > rf::kPhCount + 3) out[rf::kPhCount + 3] = lines ? 2.0 : level ? 1.0 : 0.0;
+      if (n > rf::kPhCount + 4) out[rf::kPhCount + 4] = double(lines ? c.pen.cs : level ? 1 : c.cluster_size);
+      if (n > rf::kPhCount + 5) out[rf::kPhCount + 5] = double(rf::factor_ctas(c));
     }
     if (enable >= 0) c.profiling = enable > 0;
     if (reset) {

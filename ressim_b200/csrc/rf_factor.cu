@@ -596,6 +596,8 @@ void build_factor_plan(Ctx& c) {
   P.built = 1;
 }
 
+int factor_ctas(const Ctx& c) { return !c.fac.built ? c.cluster_size : c.batched ? kFacBatchCtas : c.fac.cs; }
+
 void factor_levels(Ctx& c) {
   FactorPlan& P = c.fac;
   const long long nnzb = c.nnzb;

@@ -103,6 +103,7 @@ void launch_block_sweep_level(Ctx& c, const double* cr, double* x, const void* l
 // topology, and the launches.
 void build_factor_plan(Ctx& c);
 void free_factor_plan(Ctx& c);
+int factor_ctas(const Ctx& c);  // CTAs of a factorisation
 void factor_levels(Ctx& c);
 
 // Largest deck whose pressure stage is the dense inverse of its matrix.
