@@ -406,16 +406,24 @@ MATCHED_CNV, MATCHED_MB = 1e-8, 1e-10
 MATCHED_LIN_RTOL, MATCHED_LIN_PASSES = 1e-10, 12
 
 
-# DRAM bytes (read + write) per algorithmic byte of one batched level-order pressure launch, from
-# an ncu capture (dram__bytes_read.sum + dram__bytes_write.sum, one pass, caches flushed before the
-# launch) of the first k_bicgstab_level_batch launch of `bench.py --variants 2 --host-threads 1
-# --steps 1 --warmup 0`: variants 0 and 1 (18,705 and 39,480 cells), 50 iterations each, 11.03 MB
-# of DRAM traffic against 1,901 MB of algorithmic bytes.  The solves' working set is read from
-# DRAM about once and every later pass hits L2.
-LEVEL_BATCH_DRAM_PER_ALG_BYTE = 11.03e6 / 1901.47e6
-# DRAM bytes per launch of the one-cluster pressure BiCGStab on the 60x60x20 black-oil deck
-# (k_bicgstab_dsmem, ncu dram__bytes_read.sum + dram__bytes_write.sum, caches flushed).
-CLUSTER_DRAM_PER_LAUNCH = {"72k-bo": 15.71e6}
+# DRAM bytes (read + write) per algorithmic byte of one batched pressure launch, from an ncu capture
+# (dram__bytes_read.sum + dram__bytes_write.sum, caches flushed before the launch) of the first
+# k_bicgstab_pencil_batch launch of `bench.py --variants 2 --host-threads 1 --steps 1 --warmup 0`:
+# variants 0 and 1 (18,705 and 39,480 cells) on eight CTAs each, 50 iterations each, 13.35 MB of DRAM
+# traffic against 1,901 MB of algorithmic bytes.  The solves' working set is read from DRAM about
+# once and every later pass hits L2.
+LINES_BATCH_DRAM_PER_ALG_BYTE = 13.354e6 / 1901.47e6
+# DRAM bytes per launch of the pressure BiCGStab along grid lines on the 60x60x20 black-oil deck
+# (k_bicgstab_pencil, 16 CTAs, the same metrics).
+LINES_DRAM_PER_LAUNCH = {"72k-bo": 15.526e6}
+# Kernels of the pressure stage as the profile names them: a single deck's, and a batched launch's.
+PRESSURE_KERNELS = {
+    "lines": ("k_bicgstab_pencil (along grid lines, one thread-block cluster)",
+              "k_bicgstab_pencil_batch (one launch = a group's pressure solves, one thread-block cluster each)"),
+    "level": ("k_bicgstab_level (level order, one thread block)",
+              "k_bicgstab_level_batch (one launch = a group's pressure solves, one thread block each)"),
+    "cluster": ("k_bicgstab_dsmem / k_bicgstab_cluster (one thread-block cluster)",) * 2,
+}
 
 
 def ensemble_roofline(ds, profs, peak, peak_kind, batch=None):
@@ -430,18 +438,20 @@ def ensemble_roofline(ds, profs, peak, peak_kind, batch=None):
     byts = sum(bicgstab_bytes_per_iteration(d.n_cells, p["nnzb"]) * p["bicgstab_iterations"] for d, p in zip(ds, profs))
     if batch is not None and batch.get("pressure_launches", 0) > 0 and batch.get("pressure_ms", 0) > 0:
         nl, kms = batch["pressure_launches"], batch["pressure_ms"]
-        kernel = "k_bicgstab_level_batch (one launch = a group's pressure solves, one thread block each)"
+        batched = 1
         solves = batch["pressure_items"]
     else:
         nl = sum(p["bicgstab_launches"] for p in profs)
         kms = sum(p["bicgstab_kernel"] for p in profs)
-        kernel = "k_bicgstab_level (one launch = one variant's pressure solve, one thread block)"
+        batched = 0
         solves = nl
     if nl <= 0 or kms <= 0:
         return None
     phase_ms = sum(sum(p[k] for k in _lib.PHASES if k != "bicgstab_kernel") for p in profs)
     achieved = (byts / nl) / (kms / nl / 1e3) / 1e9
-    traffic = LEVEL_BATCH_DRAM_PER_ALG_BYTE * byts / nl
+    kinds = sorted({p["pressure_kernel"] for p in profs})
+    kernel = "; ".join(PRESSURE_KERNELS[k][batched] for k in kinds)
+    traffic = LINES_BATCH_DRAM_PER_ALG_BYTE * byts / nl if kinds == ["lines"] else None
     return {"kernel": kernel, "bound": "hbm", "achieved": achieved, "peak": peak, "peak_kind": peak_kind,
             "unit": "GB/s", "frac": achieved / peak, "traffic": traffic,
             "traffic_basis": "ncu DRAM bytes per algorithmic byte of one batched launch (caches flushed), "
@@ -1011,10 +1021,9 @@ def main():
         bytes_launch = bicgstab_bytes_per_iteration(n, nnzb) * iters / launches_b
         ms_launch = kernel_ms / launches_b
         achieved = bytes_launch / (ms_launch / 1e3) / 1e9
-        kname = ("k_bicgstab_level (one thread block, level order)" if prof.get("level_kernels")
-                 else "k_bicgstab_dsmem / k_bicgstab_cluster (one thread-block cluster)")
-        traffic = (None if prof.get("level_kernels") or args.precision != "fp64"
-                   else CLUSTER_DRAM_PER_LAUNCH.get(args.workload))
+        kname = PRESSURE_KERNELS[prof["pressure_kernel"]][0]
+        traffic = (LINES_DRAM_PER_LAUNCH.get(args.workload)
+                   if prof["pressure_kernel"] == "lines" and args.precision == "fp64" else None)
         roof = {"kernel": kname, "bound": "hbm", "achieved": achieved, "peak": peak,
                 "peak_kind": peak_kind, "unit": "GB/s", "frac": achieved / peak, "traffic": traffic,
                 "bytes_per_launch": bytes_launch, "ms_per_launch": ms_launch,
