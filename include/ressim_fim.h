@@ -231,10 +231,13 @@ int32_t rf_linear_solve_csr(RfCtx* ctx, int32_t n_rows, const int32_t* row_ptr, 
  * effect at the next linear solve. */
 int32_t rf_set_linear_precision(RfCtx* ctx, int32_t mode);
 
-/* Tuning: CTAs (1..16, rounded down to a launchable power of two) in the thread-block cluster that
- * runs the level-scheduled ILU factorisation, ILU sweeps and pressure BiCGStab; 0 restores the
- * automatic choice (enough 1024-thread CTAs for the widest level).  Returns the size in use (> 0)
- * or an error.  The size fixes the reduction order, so results are deterministic for a given size
+/* Tuning: CTAs (1..16, rounded down to a launchable power of two) of the thread-block clusters that
+ * run the ILU factorisation, the pressure BiCGStab along grid lines (the nearest size the deck
+ * fits) and the cluster kernels of the ILU sweeps and the BiCGStab; 0 restores the automatic choice,
+ * each kernel's own.  The level-order kernels run on one CTA, and the batched factorisation of
+ * RF_BATCH_GROUPS keeps its size.  Returns the cluster kernels' size (> 0) or an error; rf_profile
+ * reports the others.  Where the cluster kernels, or the solve along lines in their place, serve the
+ * pressure stage, their size fixes the reduction order: results are deterministic for a given size
  * and differ between sizes only by rounding.  No counterpart in the reference. */
 int32_t rf_set_cluster_size(RfCtx* ctx, int32_t ctas);
 

@@ -1,10 +1,11 @@
-"""Autotuner of the ensemble form: the thread-block cluster size of each variant's level-scheduled
-kernels (block-ILU0 factorisation and sweeps, the pressure BiCGStab).
+"""Autotuner of the ensemble form: the thread-block cluster size of each variant's pressure solve along
+grid lines and, outside batched launches, of its block-ILU0 factorisation; for decks that take the
+cluster kernels, of those.
 
 No counterpart in the reference, which solves one deck on one CPU thread.  The cluster size is
-the device path's one launch-shape choice: the smallest size whose slices fit the shared-memory
-form is the automatic default, while a larger cluster shortens each level step's work and a
-smaller one leaves more SMs to the other variants of a batch.
+the device path's one launch-shape choice: by default the solve takes the fewest CTAs whose lines are
+one warp's, up to a limit that falls with the ensemble's size, while a larger cluster shortens each
+step's work and a smaller one leaves more SMs to the other variants of a batch.
 
 - `tune` measures, for each candidate size, the device time of one report step of a deck from
   the same state, and persists the curve as JSON keyed by grid dimensions and precision
@@ -16,8 +17,9 @@ smaller one leaves more SMs to the other variants of a batch.
   from every variant's fastest size and moves variants to smaller clusters, best SM-time saving
   per latency added first, while that lowers the larger of the two bounds.
 - `criterion="sm_time"` (least T cs per variant) and `"latency"` (fastest per variant) keep the
-  per-variant choices; on the 256-variant ensemble the SM-time choice alone was slower than the
-  automatic sizes (312k against 526k cell-steps/s), because the batch is latency bound too.
+  per-variant choices.  On the 256-variant FP64 ensemble in batched groups (3 report steps after 3)
+  the plan's sizes (5 x 1, 38 x 2, 178 x 4, 31 x 8, 4 x 16) gave 1.58M cell-steps/s, the automatic
+  ones 1.65M: the curves are of variants that have the device for themselves.
 """
 from __future__ import annotations
 

@@ -1579,7 +1579,12 @@ int64_t rf_kernel_launches(const RfCtx* ctx) { return ctx ? ctx->c.launches : 0;
 int32_t rf_set_cluster_size(RfCtx* ctx, int32_t ctas) {
   if (!ctx || ctas < 0 || ctas > 16) return RF_ERR_INVALID;
   return guarded(ctx, [&]() -> int32_t {
-    return rf::set_cluster_size(ctx->c, ctas == 0 ? rf::auto_cluster_size(ctx->c) : ctas);
+    rf::Ctx& c = ctx->c;
+    const int used = rf::set_cluster_size(c, ctas == 0 ? rf::auto_cluster_size(c) : ctas);
+    c.cluster_fixed = ctas == 0 ? 0 : used;
+    rf::factor_fix(c);
+    rf::pencil_replan(c);
+    return used;
   });
 }
 

@@ -128,7 +128,7 @@ struct PencilPlan {
 
 // Plan of the ILU0 factorisations (rf_factor.cu): simple rows and listed rows' steps by level.
 struct FactorPlan {
-  int built = 0, cs = 1;  // cs: CTAs of a single deck's factorisation
+  int built = 0, cs = 1, fixed = 0;  // CTAs of a single deck's factorisation, automatic and asked for (0: not)
   DBuf<int> d_row_ptr, d_step_ptr;
   DBuf<int4> d_rec, d_step, d_entry;
   DBuf<int2> d_pair;
@@ -249,6 +249,7 @@ struct Ctx {
   // discrete adjoint tape (rf_adjoint.cu); null until recording starts
   struct AdjointTape* tape = nullptr;
   int cluster_size = 0;  // CTAs in the one cluster that runs the level-scheduled kernels
+  int cluster_fixed = 0;  // that size where rf_set_cluster_size asked for one (0: automatic)
   // slice ownership schedule of the distributed-shared-memory BiCGStab (built for cluster_size)
   int own_slice = 0;
   size_t dsm_bytes[2] = {0, 0};  // dynamic shared memory per CTA for double / float; 0: does not fit

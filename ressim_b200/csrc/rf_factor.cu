@@ -596,7 +596,12 @@ void build_factor_plan(Ctx& c) {
   P.built = 1;
 }
 
-int factor_ctas(const Ctx& c) { return !c.fac.built ? c.cluster_size : c.batched ? kFacBatchCtas : c.fac.cs; }
+int factor_ctas(const Ctx& c) {
+  if (!c.fac.built) return c.cluster_size;
+  return c.batched ? kFacBatchCtas : c.fac.fixed ? c.fac.fixed : c.fac.cs;
+}
+
+void factor_fix(Ctx& c) { c.fac.fixed = c.cluster_fixed == 16 && !fac_sixteen() ? 8 : c.cluster_fixed; }
 
 void factor_levels(Ctx& c) {
   FactorPlan& P = c.fac;
@@ -620,7 +625,7 @@ void factor_levels(Ctx& c) {
   a.pdiag = c.d_pdiag.p;
   if (!(c.batched && fiber_file(kBatchFactor, 0, &a, sizeof(a), kFacThreads, 0))) {
     void* args[] = {&a};
-    RF_CUDA(fac_launch((const void*)k_factor_levels, 1, P.cs, args, c.stream));
+    RF_CUDA(fac_launch((const void*)k_factor_levels, 1, P.fixed ? P.fixed : P.cs, args, c.stream));
     c.launches++;
   }
   k_factor_post<<<(c.n + kBlock - 1) / kBlock, kBlock, 0, c.stream>>>(

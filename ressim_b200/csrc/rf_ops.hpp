@@ -104,6 +104,7 @@ void launch_block_sweep_level(Ctx& c, const double* cr, double* x, const void* l
 void build_factor_plan(Ctx& c);
 void free_factor_plan(Ctx& c);
 int factor_ctas(const Ctx& c);  // CTAs of a factorisation
+void factor_fix(Ctx& c);        // takes over c.cluster_fixed
 void factor_levels(Ctx& c);
 
 // Largest deck whose pressure stage is the dense inverse of its matrix.

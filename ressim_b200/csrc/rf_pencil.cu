@@ -1266,13 +1266,14 @@ bool pen_cs_fits(Ctx& c, int cs) {
 // 181 / 202, 40x31x5 267 / 203 / 197 / 221, 45x61x7 789 / 429 / 388 / 381, 60x60x20 - / 1067 / 764 /
 // 618.  An ensemble's variants share the chip: at most 8 CTAs each for up to 32 variants, 4 beyond
 // (a report step of 16 variants on 4 / 8 / 16 CTAs: 407 / 374 / 493 ms, of 32: 1006 / 962 / 1260, of
-// 64: 1361 / 1479 / 2204).
+// 64: 1361 / 1479 / 2204).  A size that rf_set_cluster_size asked for is taken where the deck fits it.
 int pencil_want(Ctx& c) {
   PencilPlan& P = c.pen;
   const int f = c.precision == 1 ? 1 : 0;
   const int most = c.ensemble == 0 ? 16 : c.ensemble <= 32 ? 8 : 4;
   int want = 1;
   while (want < most && c.nz * ((c.ny + want - 1) / want) > 32) want *= 2;
+  if (c.cluster_fixed > 0) want = c.cluster_fixed;
   auto fits = [&](int k) {
     int& v = P.fits[f][k];
     if (v < 0) v = (f == 1 ? pen_cs_fits<float>(c, 1 << k) : pen_cs_fits<double>(c, 1 << k)) ? 1 : 0;

@@ -162,8 +162,9 @@ class ReservoirSimulator(Deck):
             raise DeviceError(f"rf_set_linear_precision failed ({rc}): {_lib.last_error(self._context())}")
 
     def set_cluster_size(self, ctas: int = 0) -> int:
-        """CTAs of the cluster running the level-scheduled kernels (0: automatic); returns the size
-        in use."""
+        """CTAs of the clusters running the factorisation, the pressure solve along grid lines and the
+        cluster kernels (0: automatic, each its own); returns the cluster kernels' size.  `profile`
+        has the others as factor_ctas and pressure_ctas."""
         rc = _lib.load().rf_set_cluster_size(self._context(), int(ctas))
         if rc <= 0:
             raise DeviceError(f"rf_set_cluster_size failed ({rc}): {_lib.last_error(self._context())}")
