@@ -112,9 +112,9 @@ struct PencilPlan {
   int lost_message = -1;  // PenArgs::lost
   int typed = -1;       // value type the buffers hold (-1: zeros, which serve either)
   struct Listed {
-    int j, entries;
+    int j, ik, entries;
   };
-  std::vector<Listed> listed;               // rows taken from lists: column, entries off the diagonal
+  std::vector<Listed> listed;               // rows taken from lists: column, i + k, entries off the diagonal
   std::set<std::pair<int, int>> fill_cols;  // columns (j, j') joined by a well's fill
   std::vector<int> h_spec_row, h_spec_col_row, h_nat, dots_key;  // dots_key: the order d_list holds
   DBuf<int> d_cta, d_nat, d_rec_at, d_rec_half, d_list_ptr, d_list[3], d_spec_slot, d_spec_ptr, d_spec_col, d_spec_map;

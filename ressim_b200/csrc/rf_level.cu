@@ -1008,9 +1008,14 @@ void level_plan_reshape(Ctx& c) {
 // quickly (measured crossover between 19k and 40k cells).
 constexpr int kLevelAutoCells = 32768;
 
+static bool level_size(const Ctx& c) { return c.batched || c.n <= kLevelAutoCells; }
 static bool level_chosen(const Ctx& c) {
   if (c.pressure_solver == 2) return true;
-  return c.pressure_solver == 0 && (c.batched || c.n <= kLevelAutoCells);
+  return c.pressure_solver == 0 && level_size(c);
+}
+
+bool level_automatic(const Ctx& c) {
+  return c.lvl.built && c.lvl.fits[c.precision == 1 ? 1 : 0] && level_size(c);
 }
 
 bool level_solver_active(const Ctx& c) {

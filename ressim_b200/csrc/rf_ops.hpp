@@ -95,6 +95,7 @@ void free_level_plan(Ctx& c);
 void level_plan_reshape(Ctx& c);
 bool level_solver_active(const Ctx& c);
 bool level_block_sweep_active(const Ctx& c);
+bool level_automatic(const Ctx& c);  // the automatic choice takes them, but for the solve along lines
 void level_pack(Ctx& c);
 void launch_bicgstab_level(Ctx& c, const double* rhs, double* x);
 void launch_block_sweep_level(Ctx& c, const double* cr, double* x, const void* lu, const void* dinv);

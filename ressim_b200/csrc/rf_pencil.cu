@@ -35,8 +35,9 @@
 // cluster size or the thread count here, so results equal those kernels' bit for bit.
 //
 // Used when every cell's level is i+j+k (no well fill deepens the levels), each well's fill stays
-// within one CTA's columns and the padding of the step order stays small; other decks, and callers
-// that name a kernel family, keep the level-list kernels.
+// within one CTA's columns, the padding of the step order stays small and the wells' rows do not crowd
+// the chain of steps (pen_crowded); other decks, and callers that name a kernel family, keep the
+// level-list kernels.
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
@@ -1260,6 +1261,41 @@ bool pen_cs_fits(Ctx& c, int cs) {
   return true;
 }
 
+// The most listed rows on one chain of a forward sweep's steps, through the CTAs: a step comes after the
+// CTA's step before and the step that sends it the neighbour's column.
+int pen_listed_path(const Ctx& c, int cs) {
+  std::vector<int> before, path;
+  int cols_before = 0;
+  for (int b = 0; b < cs; ++b) {
+    const int first = pen_first_col(b, cs, c.ny), cols = pen_first_col(b + 1, cs, c.ny) - first;
+    path.assign(pen_steps(c.nx, cols, c.nz), 0);
+    for (const PencilPlan::Listed& r : c.pen.listed)
+      if (r.j >= first && r.j < first + cols) path[r.ik + r.j - first]++;
+    for (int m = 0; m < int(path.size()); ++m) {
+      int at = m > 0 ? path[m - 1] : 0;
+      if (b > 0) at = std::max(at, before[std::min(m + cols_before, int(before.size()) - 1)]);
+      path[m] += at;
+    }
+    before.swap(path);
+    cols_before = cols;
+  }
+  return before.back();
+}
+
+// Whether the level-order kernel is the faster one for the deck's wells.  A step's listed rows are solved
+// one after another, 1.6 us each per iteration where they lie on one chain of steps; the level-order
+// kernel spreads a level's rows over its threads and takes 2.6-4.3 us per level and iteration, the solve
+// along lines 1.0-1.8 us besides the listed rows.  us per iteration along lines / in level order, wells through
+// all layers (FP64; FP32 alike): 10x10x5 with 2 / 8 / 23 wells (10 / 38 / 97 rows on a chain, 23 levels)
+// 54 / 64, 94 / 76, 179 / 87; 20x20x5 with 8 / 23 / 58 (30 / 65 / 162, 43) 98 / 143, 149 / 154, 293 / 167;
+// 16x64x16 with 8 / 16 / 24 (90 / 163 / 229, 94) 261 / 367, 385 / 383, 494 / 399; 64x64x8 with 112 (223, 134)
+// 476 / 579.  The cluster kernels are slower than it throughout (36,000 to 80,000 cells, chains of up to
+// 3.4 rows per level: 1.9-3.6 times).
+bool pen_crowded(const Ctx& c, int cs) {
+  if (!level_automatic(c)) return false;
+  return 10 * pen_listed_path(c, cs) > 17 * c.levels.n_levels - 130;
+}
+
 // CTAs per solve: the fewest whose columns are one warp's lines (a warp's barrier is 15 cycles, 13
 // warps' 45, and a step's rows come from L2 over more SMs; each hand-over to the next CTA costs some
 // 100 cycles of a step).  Thousand cycles per iteration on 1 / 4 / 8 / 16 CTAs: 21x20x5 211 / 173 /
@@ -1280,11 +1316,13 @@ int pencil_want(Ctx& c) {
     return v > 0;
   };
   const int k0 = log2_of(want);
-  for (int k = k0; k >= 0; --k)
-    if (fits(k)) return 1 << k;
-  for (int k = k0 + 1; k < 5; ++k)
-    if (fits(k)) return 1 << k;
-  return 0;
+  int k = k0;
+  while (k >= 0 && !fits(k)) --k;
+  if (k < 0) {
+    k = k0 + 1;
+    while (k < 5 && !fits(k)) ++k;
+  }
+  return k < 5 && !pen_crowded(c, 1 << k) ? 1 << k : 0;
 }
 
 template <class V, class H>
@@ -1496,7 +1534,7 @@ bool pencil_structure(Ctx& c) {
   for (int r = 0; r < n; ++r) {
     if (!special[r]) continue;
     P.h_spec_row.push_back(r);
-    P.listed.push_back({(r / nx) % ny, c.h_row_ptr[r + 1] - c.h_row_ptr[r] - 1});
+    P.listed.push_back({(r / nx) % ny, r % nx + r / (nx * ny), c.h_row_ptr[r + 1] - c.h_row_ptr[r] - 1});
     for (int e = c.h_row_ptr[r]; e < c.h_row_ptr[r + 1]; ++e) {
       P.h_spec_col_row.push_back(c.h_col[e]);
       spec_map.push_back(e);
