@@ -1600,6 +1600,7 @@ int32_t rf_set_pressure_solver(RfCtx* ctx, int32_t kind, int32_t threads) {
     c.pressure_solver = kind;
     c.level_threads = threads;
     rf::level_plan_reshape(c);
+    rf::pencil_replan(c);  // the sums' order, and the choice against the level-order kernels, follow its threads
     if (kind == RF_PRESSURE_SOLVER_LEVEL && !c.lvl.fits[c.precision == 1 ? 1 : 0]) {
       c.err = "the level-order pressure solver's window does not fit shared memory on this device";
       c.pressure_solver = RF_PRESSURE_SOLVER_AUTO;

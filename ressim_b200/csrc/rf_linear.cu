@@ -2318,7 +2318,7 @@ LinResult linear_solve_full(Ctx& c, std::vector<double>& h_dx_tail) {
 }
 
 // ---- one-time setup ----
-// Update lists of the factorisation (FacRecipes) for the current pattern.
+// Level schedule of the lower block pattern.
 void build_levels(Ctx& c) {
   const int n = c.n;
   std::vector<int> lvl(n, 0);
@@ -2605,8 +2605,9 @@ void setup_linear_workspace(Ctx& c) {
   set_cluster_size(c, auto_cluster_size(c));
   build_level_plan(c);
   build_pencil_plan(c);
-  // RESSIM_FACTOR_RECIPES=0 (read when a context is set up) keeps the searching form of the
-  // factorisation; the two give identical factors, which the tests check through it
+  // RESSIM_FACTOR_RECIPES=0 (read when a context is set up; the name is from the update lists that the
+  // plan took the place of) keeps the searching form of the factorisation; the two give identical factors,
+  // which the tests check through it
   const char* env = std::getenv("RESSIM_FACTOR_RECIPES");
   if (!env || std::strcmp(env, "0") != 0) build_factor_plan(c);
   const int nt = 1 + c.topo.max_perfs_per_well;
