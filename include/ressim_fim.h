@@ -248,8 +248,8 @@ int32_t rf_set_cluster_size(RfCtx* ctx, int32_t ctas);
  * 32..512 in steps of 32, 0 automatic); RF_PRESSURE_SOLVER_AUTO (default) takes the level-order
  * kernels, where their level window fits shared memory, for decks of up to 32,768 cells and for
  * every variant of an ensemble stepped in RF_BATCH_GROUPS mode, and the cluster kernels otherwise;
- * its pressure BiCGStab runs along grid lines where the deck allows, with the results of the kernel
- * it stands in for bit for bit.  All compute the same preconditioner; the cluster's and the level
+ * its pressure BiCGStab runs along grid lines where the deck allows and that is the faster kernel, with
+ * the results of the kernel it stands in for bit for bit.  All compute the same preconditioner; the cluster's and the level
  * order's solves differ only in the summation order of their dot products.  Takes effect at the next
  * linear solve; RF_ERR_UNSUPPORTED when the level-order kernels cannot run this deck.  No
  * counterpart in the reference. */

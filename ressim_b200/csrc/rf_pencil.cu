@@ -1290,7 +1290,7 @@ int pen_listed_path(const Ctx& c, int cs) {
 // 54 / 64, 94 / 76, 179 / 87; 20x20x5 with 8 / 23 / 58 (30 / 65 / 162, 43) 98 / 143, 149 / 154, 293 / 167;
 // 16x64x16 with 8 / 16 / 24 (90 / 163 / 229, 94) 261 / 367, 385 / 383, 494 / 399; 64x64x8 with 112 (223, 134)
 // 476 / 579.  The cluster kernels are slower than it throughout (36,000 to 80,000 cells, chains of up to
-// 3.4 rows per level: 1.9-3.6 times).
+// 3.4 rows per level: 1.9-3.8 times).
 bool pen_crowded(const Ctx& c, int cs) {
   if (!level_automatic(c)) return false;
   return 10 * pen_listed_path(c, cs) > 17 * c.levels.n_levels - 130;
@@ -1302,7 +1302,7 @@ bool pen_crowded(const Ctx& c, int cs) {
 // 181 / 202, 40x31x5 267 / 203 / 197 / 221, 45x61x7 789 / 429 / 388 / 381, 60x60x20 - / 1067 / 764 /
 // 618.  An ensemble's variants share the chip: at most 8 CTAs each for up to 32 variants, 4 beyond
 // (a report step of 16 variants on 4 / 8 / 16 CTAs: 407 / 374 / 493 ms, of 32: 1006 / 962 / 1260, of
-// 64: 1361 / 1479 / 2204).  A size that rf_set_cluster_size asked for is taken where the deck fits it.
+// 64: 1361 / 1479 / 2204; fewer CTAs, and more variants, were not timed).  A size that rf_set_cluster_size asked for is taken where the deck fits it.
 int pencil_want(Ctx& c) {
   PencilPlan& P = c.pen;
   const int f = c.precision == 1 ? 1 : 0;
