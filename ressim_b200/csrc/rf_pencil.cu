@@ -1302,7 +1302,8 @@ bool pen_crowded(const Ctx& c, int cs) {
 // 181 / 202, 40x31x5 267 / 203 / 197 / 221, 45x61x7 789 / 429 / 388 / 381, 60x60x20 - / 1067 / 764 /
 // 618.  An ensemble's variants share the chip: at most 8 CTAs each for up to 32 variants, 4 beyond
 // (a report step of 16 variants on 4 / 8 / 16 CTAs: 407 / 374 / 493 ms, of 32: 1006 / 962 / 1260, of
-// 64: 1361 / 1479 / 2204; fewer CTAs, and more variants, were not timed).  A size that rf_set_cluster_size asked for is taken where the deck fits it.
+// 64: 1361 / 1479 / 2204; fewer CTAs, and more variants, were not timed).  A size that
+// rf_set_cluster_size asked for is taken where the deck fits it.
 int pencil_want(Ctx& c) {
   PencilPlan& P = c.pen;
   const int f = c.precision == 1 ? 1 : 0;
