@@ -159,6 +159,11 @@ __device__ __forceinline__ int lds_i(unsigned a) {
   asm volatile("ld.shared.s32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
   return v;
 }
+__device__ __forceinline__ int2 lds_i2(unsigned a) {
+  int2 v;
+  asm volatile("ld.shared.v2.s32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a) : "memory");
+  return v;
+}
 __device__ __forceinline__ void sts(unsigned a, double v) {
   asm volatile("st.shared.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
 }
@@ -383,7 +388,8 @@ __device__ __noinline__ void pen_load(const PenSweep<T>& w, unsigned phase0, con
   const unsigned recs = w.place, ins = recs + unsigned(2 * G) * 4u * RB, rds = ins + unsigned(2 * G) * RB;
   const unsigned cb = unsigned(G) * RB, db = 8u * unsigned(G) * unsigned(stride);
   // chunk number c of the sweep covers the rows [G k, G k + G), k = c or, backward, from the end
-  bool ok = lds_i(w.gave) == 0;  // the same for all lanes
+  // the same for all lanes; no forward sweep starts after a wait gave up
+  bool ok = FWD || lds_i(w.gave) == 0;
   unsigned open = 0;             // the halves whose copies have not been waited for
   auto issue = [&](int c) {
     if (!ok || c >= chunks) return;
@@ -1015,18 +1021,20 @@ __device__ void pen_body(const PenArgs<T>& a, unsigned char* raw) {
         __syncthreads();
         // any CTA's flags reach all of them.  `bad`: the sweep is repeated, and the solve goes on, in
         // the general form; `gave`: the solve ends
-        if (tid < g.cs) {
-          if (!general && lds_i(bad_at) != 0)
+        const int2 own = lds_i2(bad_at);
+        if ((own.x | own.y) != 0 && tid < g.cs) {
+          if (!general && own.x != 0)
             asm volatile("st.shared::cluster.s32 [%0], 1;" ::"r"(pen_map(bad_at, unsigned(tid))) : "memory");
-          if (lds_i(gave_at) != 0)
+          if (own.y != 0)
             asm volatile("st.shared::cluster.s32 [%0], 1;" ::"r"(pen_map(gave_at, unsigned(tid))) : "memory");
         }
         pen_sync(g.cs);
-        if (lds_i(gave_at) != 0) {
+        const int2 any = lds_i2(bad_at);
+        if (any.y != 0) {
           stop = true;
           break;
         }
-        if (general || lds_i(bad_at) == 0) break;
+        if (general || any.x == 0) break;
         general = true;
         pen_clear(sweep[1]);  // the attempt may have left NaNs: pen_div of a pivot that pen_recip refuses
         __syncthreads();

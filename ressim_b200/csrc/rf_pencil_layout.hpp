@@ -52,7 +52,7 @@ RF_PEN_HD inline PenLayout pen_layout(int nx, int nz, int cols, int cs, int chun
   o.mbar = take(cs > 1 ? 2 * size_t(nx + nz - 1) * 8 : 0);
   o.full = take(2 * 8);
   o.red = take(4 * size_t(nvw) * sizeof(double));
-  o.bad = take(2 * sizeof(int));  // two flags
+  o.bad = take(2 * sizeof(int));  // two flags, read together
   // The places above are the same in every CTA of a cluster: CTAs store to one another's by their own
   // offsets (nbr, mbar, red, bad).  Below, each CTA's own wells.
   o.well_in = take(size_t(wells) * sizeof(T));
