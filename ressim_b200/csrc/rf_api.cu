@@ -1658,7 +1658,8 @@ int32_t rf_profile(RfCtx* ctx, int32_t enable, int32_t reset, double* out, int32
 //    launch per kind (rf_fiber.cu);
 //  - RF_BATCH_THREADS: one stream per variant and a pool of host threads, each stepping one
 //    variant at a time with its own launches.
-// The variants never exchange data, and a variant's results are the same either way.
+// The variants never exchange data, and a variant's results are the same either way (above 32,768 cells
+// to rounding: the groups' pressure solves keep the level order's sums there too).
 // ---------------------------------------------------------------------------------------------
 struct RfBatch {
   std::vector<RfCtx*> ctx;
